@@ -10,8 +10,11 @@
 // carry with a transfer matrix fixed by the factors (precomputed on the host), so each sweep runs
 // in three phases:
 //   A: every chunk sweeps with a zero incoming carry and records its outgoing carry;
-//   B: a log-depth scan over the chunks chains the carries through products of transfer matrices;
+//   B: the carries are chained through the transfer matrices: from the few chunks whose carries
+//      still reach (carry_direct), or, where the transfers decay slowly, by a log-depth scan;
 //   C: every chunk sweeps again from its true carry and writes its rows.
+// reg_solve.cuh holds the same solve with a chunk's rows in registers, in the same order of
+// operations: both give the same bits.
 // Periodic systems add a border of k rows/cols (Schur complement; the 2x2 block solve of
 // splines_linear_problem_2x2_blocks.cpp:274-298) applied in shared memory.
 #pragma once
@@ -51,10 +54,6 @@ __device__ __forceinline__ int64_t tile_line0(BuildArgs const& args)
 }
 
 
-__device__ __forceinline__ int64_t line_offset(Lines const& L, int64_t b)
-{
-    return (b / L.inner) * L.outer_stride + (b % L.inner);
-}
 
 __device__ __forceinline__ void cp_async8(void* smem_dst, const void* gmem_src)
 {
@@ -132,22 +131,23 @@ __device__ __forceinline__ V zero_of() { return V {}; }
 
 // Forward sweep with L (and the row interchanges when PIV) over rows [a, e) (chunk c) of a line
 // pair (or of the single line); T2 points at the pair's column (row j at T2[j*P]). w[0..KL-1] hold rows a..a+KL-1 on
-// entry. Phase A (WRITE false) reads rows beyond e from the tile, which nothing has written yet.
-// Phase C (WRITE true) writes rows a..e-1; without interchanges rows beyond e only feed the next
-// chunk's rows, so they are not read; with interchanges they come from the halo copy.
+// entry. Without interchanges rows beyond e only feed the next chunk's rows, so they count as 0 and
+// the window ends as the outgoing carry. With interchanges phase A (WRITE false) reads them from the
+// tile, which nothing has written yet, and phase C (WRITE true) from the halo copy. Phase C writes
+// rows a..e-1.
 template <class R, class V, int KL, bool PIV, bool WRITE, int UNR>
 __device__ __forceinline__ void fwd_sweep(SolveTables const& t, V* T2, int P, int a, int e, int c, V* w, const V* halo,
                                           int hstride)
 {
     R const* __restrict__ Lf = Fac<R>::Lf(t);
-    int const lim = (WRITE && !PIV) ? e : t.m; // fill rows below lim are read
+    int const lim = PIV ? t.m : e; // fill rows below lim are read
     int const qs = factor_stride(t);
 #pragma unroll UNR
     for (int j = a; j < e; ++j) {
         int const rr = j + KL;
         V fill = zero_of<V>();
         if (rr < e) fill = T2[rr * P];
-        else if (rr < lim) fill = (WRITE && PIV) ? halo[(rr - e) * hstride] : T2[rr * P];
+        else if (rr < lim) fill = WRITE ? halo[(rr - e) * hstride] : T2[rr * P];
         w[KL] = fill;
         if (PIV) {
             int const pv = __ldg(t.piv + piv_index(t, j, a, c));
@@ -181,12 +181,41 @@ __device__ __forceinline__ void bwd_sweep(SolveTables const& t, V* T2, int P, in
         R const* U = Uf + factor_base(t, j, a, c, KU + 1);
         V s = T2[j * P];
 #pragma unroll
-        for (int q = 1; q <= KU; ++q) s = fma2(-__ldg(U + q * qs), z[q - 1], s);
+        for (int q = KU; q >= 1; --q) s = fma2(-__ldg(U + q * qs), z[q - 1], s); // the newest row last: a short chain
         V const x = mul2(s, __ldg(U));
         if (WRITE) T2[j * P] = x;
 #pragma unroll
         for (int q = KU - 1; q >= 1; --q) z[q] = z[q - 1];
         z[0] = x;
+    }
+}
+
+// The true carry leaving chunk b in the sweep's direction (forward: b and the chunks before it,
+// backward: b and those after it), from the outgoing carries C2 of the nd <= kDirectCarry chunks
+// that end with b:
+//   y(b) = hat(b) + Phi_b (hat(b-1) + Phi_{b-1} (hat(b-2) + ..)).
+// Products of nd transfers are below 2^-60, so chunks further away change no carry. A handful of
+// multiply-adds per chunk and no barrier, against two barriers per step of the scan.
+// phi(c, e): entry e (row-major) of the transfer matrix of chunk c.
+template <class V, int K, int KC, bool FWD, class Phi>
+__device__ __forceinline__ void carry_direct(Phi phi, const V* C2, int P, int nd, int NC, int b, V* acc)
+{
+    int const t0 = min(nd - 1, FWD ? b : NC - 1 - b); // the furthest chunk of the line that still reaches b
+    int nb = FWD ? b - t0 : b + t0;
+#pragma unroll
+    for (int q = 0; q < K; ++q) acc[q] = C2[(nb * KC + q) * P];
+#pragma unroll 2
+    for (int t = 0; t < t0; ++t) {
+        nb += FWD ? 1 : -1;
+        V v[K];
+#pragma unroll
+        for (int r = 0; r < K; ++r) {
+            v[r] = C2[(nb * KC + r) * P];
+#pragma unroll
+            for (int q = 0; q < K; ++q) v[r] = fma2(phi(nb, r * K + q), acc[q], v[r]);
+        }
+#pragma unroll
+        for (int q = 0; q < K; ++q) acc[q] = v[q];
     }
 }
 
@@ -238,6 +267,22 @@ __device__ __forceinline__ void carry_scan(const R* __restrict__ Pm, V* C2, int 
         }
         __syncthreads();
     }
+}
+
+// The true carry leaving chunk b (0 outside the line): read where the scan has left it (nd = 0), or
+// chained here from its neighbours' outgoing carries.
+template <class R, class V, int K, int KC, bool FWD>
+__device__ __forceinline__ void carry_of(const R* __restrict__ Pm, const V* C2, int P, int nd, int NC, int b, V* out)
+{
+#pragma unroll
+    for (int q = 0; q < K; ++q) out[q] = zero_of<V>();
+    if (b < 0 || b >= NC) return;
+    if (nd > 0) {
+        carry_direct<V, K, KC, FWD>([&](int c, int e) { return __ldg(Pm + e * NC + c); }, C2, P, nd, NC, b, out);
+        return;
+    }
+#pragma unroll
+    for (int q = 0; q < K; ++q) out[q] = C2[(b * KC + q) * P];
 }
 
 // Shared-memory doubles of one tile: the rows, the carries, the halo rows (row interchanges only)
@@ -308,19 +353,25 @@ __device__ __forceinline__ void solve_in_tile(SolveTables const& t, int /*nct*/,
             else fwd_sweep<R, V, KL, false, false, UNR>(t, T2, P, a, e, c, w, nullptr, 0);
 #pragma unroll
             for (int q = 0; q < KL; ++q) {
-                V const orig = (e + q < m) ? T2[(e + q) * P] : zero;
-                carry[(c * KC + q) * P] = sub2(w[q], orig);
-                if (t.pivot) halo[(c * KL + q) * P] = orig;
+                V out = w[q];
+                if (t.pivot) {
+                    V const orig = (e + q < m) ? T2[(e + q) * P] : zero;
+                    out = sub2(out, orig);
+                    halo[(c * KL + q) * P] = orig;
+                }
+                carry[(c * KC + q) * P] = out;
             }
         }
         __syncthreads();
-        carry_scan<R, V, KL, KC, true, PRE>(Fac<R>::PhiF(t), carry, P, t.nscan_f, NC, c);
+        V in[KL];
+        if (t.ndep_f == 0) carry_scan<R, V, KL, KC, true, PRE>(Fac<R>::PhiF(t), carry, P, t.nscan_f, NC, c);
+        carry_of<R, V, KL, KC, true>(Fac<R>::PhiF(t), carry, P, t.ndep_f, NC, c - 1, in);
         if (c < NC) {
             V w[KL + 1];
 #pragma unroll
             for (int q = 0; q < KL; ++q) {
                 V v = (a + q < m) ? T2[(a + q) * P] : zero;
-                if (c > 0 && a + q < m) v = add2(v, carry[((c - 1) * KC + q) * P]);
+                if (c > 0 && a + q < m) v = add2(v, in[q]);
                 w[q] = v;
             }
             if (t.pivot) fwd_sweep<R, V, KL, true, true, UNR>(t, T2, P, a, e, c, w, halo + (size_t)c * KL * P, P);
@@ -338,11 +389,10 @@ __device__ __forceinline__ void solve_in_tile(SolveTables const& t, int /*nct*/,
             for (int q = 0; q < KU; ++q) carry[(c * KC + q) * P] = z[q];
         }
         __syncthreads();
-        carry_scan<R, V, KU, KC, false, PRE>(Fac<R>::PhiB(t), carry, P, t.nscan_b, NC, c);
+        if (t.ndep_b == 0) carry_scan<R, V, KU, KC, false, PRE>(Fac<R>::PhiB(t), carry, P, t.nscan_b, NC, c);
         if (c < NC) {
             V z[KU];
-#pragma unroll
-            for (int q = 0; q < KU; ++q) z[q] = (c + 1 < NC) ? carry[((c + 1) * KC + q) * P] : zero;
+            carry_of<R, V, KU, KC, false>(Fac<R>::PhiB(t), carry, P, t.ndep_b, NC, c + 1, z);
             bwd_sweep<R, V, KU, true, UNR>(t, T2, P, a, e, c, z);
         }
         __syncthreads();

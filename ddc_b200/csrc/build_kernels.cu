@@ -99,6 +99,7 @@ int pick_nct(SolveTables const& t, int TL)
 
 } // namespace
 
+bool launch_reg_build(BuildArgs const& args, cudaStream_t s);
 bool launch_build_eval_fused(BuildArgs const& args, Evaluator const& e, int order, double* out, Lines const& lo,
                              double const* coords, Lines const& lx, cudaStream_t s);
 bool launch_advect_fused(BuildArgs const& args, Evaluator const& e, double const* pts, double dt, double const* velocity,
@@ -219,6 +220,7 @@ void launch_build(Builder const& b, double* coefs, Lines const& lc, double const
     args.pair16 = line_pairs_aligned(vals, lv);
     args.pair16_out = line_pairs_aligned(coefs, lc);
     if (args.nlines == 0) return;
+    if (b.precision == DDCB_FP64 && launch_reg_build(args, s)) return;
     // long lines: fewer lines per tile, so that the tile fits in shared memory
     int const kl = b.tables.kl, ku = b.tables.ku;
     int TL;
@@ -253,6 +255,7 @@ void launch_solve_multirhs(Builder const& b, double* rhs, long ld, long nrhs, bo
     args.nct = pick_nct(args.t, b.tile_lines);
     args.pair16 = args.pair16_out = line_pairs_aligned(rhs, L);
     if (nrhs == 0) return;
+    if (launch_reg_build(args, s)) return;
     int const TL = fit_tile_lines(b.tile_lines, [&](int w) { return sizeof(double) * tile_doubles(args.t, w, args.t.kl, args.t.ku); });
     args.nct = pick_nct(args.t, TL);
     dispatch(args, TL, s);

@@ -35,6 +35,20 @@ struct Lines
     int64_t nlines() const { return inner * outer; }
 };
 
+#if defined(__CUDACC__)
+// Offset of line b. One run of lines, and lines of their own (inner = 1), need no division; the
+// others divide in 32 bits where the numbers allow (a 64-bit division costs tens of instructions).
+__device__ __forceinline__ int64_t line_offset(Lines const& L, int64_t b)
+{
+    if (L.outer <= 1) return b;
+    if (L.inner == 1) return b * L.outer_stride;
+    int64_t q;
+    if (((b | L.inner) >> 31) == 0) q = static_cast<unsigned>(b) / static_cast<unsigned>(L.inner);
+    else q = b / L.inner;
+    return q * L.outer_stride + (b - q * L.inner);
+}
+#endif
+
 inline Lines to_lines(ddcb_lines const& l) { return Lines {l.n, l.stride, l.inner, l.outer, l.outer_stride}; }
 
 // Whether lines (2i, 2i+1) of a layout sit side by side at 16-byte aligned addresses, so a tile
@@ -68,6 +82,8 @@ struct SolveTables
     const double* Lf;    // per row j, kl entries: multiplier t-1 of row j+t at step j
     const int8_t* piv;   // per row j: pivot row offset at step j (ipiv[j] - j)
     const double* Uf;    // per row j, ku+1 entries: [1/U_jj, U_j,j+1 .. U_j,j+ku]
+    int ndep_f, ndep_b;  // chunks whose outgoing carries reach a chunk's incoming one: products of
+                         // this many transfers are below 2^-60 (0: more than kDirectCarry, scan instead)
     const double* PhiF;  // transfer over chunks c-2^k+1..c (forward), kl x kl, at scan_index
     const double* PhiB;  // transfer over chunks c..c+2^k-1 (backward), ku x ku, at scan_index
     // border (k > 0)
@@ -83,6 +99,19 @@ struct SolveTables
     {
         const float *Lf, *Uf, *PhiF, *PhiB, *lam_val, *Sinv, *Qg;
     } f32;
+    // Everything the register solve (reg_solve.cuh) reads of a chunk, in one record of
+    // RegRecord<k> per chunk (copied to shared memory). rmax: rows of the longest chunk, at most
+    // kRegRows; 0: no register solve (row interchanges, wider bands, longer chunks, carries that
+    // reach further than kDirectCarry chunks).
+    const double* reg;
+    int rmax;
+    // Its border step: lambda reads rows [0, lam_lo) and [m - lam_hi, m) of Q (the ends, numbered
+    // one after the other); Q^-1 gamma corrects rows of the first cor_lo and the last cor_hi chunks.
+    // regb: one block of reg_border_size doubles: for each of those chunks and each border column
+    // kRegRows + 1 entries of Q^-1 gamma, then S^-1, lambda's values, and (as ints) its row
+    // pointers and the end row of each value.
+    int lam_lo, lam_hi, cor_lo, cor_hi;
+    const double* regb;
     // the system matrix itself in the kernel's row / column order, CSR (FP64 residuals)
     const int* a_row;    // n+1
     const int* a_col;
@@ -94,6 +123,34 @@ struct SolveTables
     double refine_tol;
     unsigned* status;
 };
+
+// A chunk's incoming carry comes straight from the outgoing carries of at most this many chunks
+// before it (no scan, no barrier); slower decays run the log-depth scan.
+constexpr int kDirectCarry = 6;
+constexpr int kRegRows = 17;       // rows of one chunk that a thread holds in registers
+constexpr int kRegMaxChunks = 128; // chunks of the longest line the register solve takes: tiles of
+                                   // eight lines (four pairs) within 512 threads
+constexpr size_t kRegSmem = 227 * 1024; // shared memory of a block on sm_100a
+// Layout (in doubles) of a chunk's record for a band of K sub- and super-diagonals: row s of the
+// chunk's L at s * LW and of its U (reciprocal diagonal first) at U + s * UW, then the transfer
+// matrices. Entries are padded to 16-byte vectors, and records are an odd number of vectors long,
+// so that the neighbouring chunks of a warp read different banks.
+struct RegRecord
+{
+    int LW, UW, U, F, B, size;
+    DDCB_HD constexpr explicit RegRecord(int K)
+        : LW(K == 3 ? 4 : K), UW((K + 2) / 2 * 2), U((kRegRows * LW + 1) / 2 * 2), F(U + kRegRows * UW), B(F + (K * K + 1) / 2 * 2),
+          size((B + (K * K + 1) / 2 * 2) / 2 % 2 ? B + (K * K + 1) / 2 * 2 : B + (K * K + 1) / 2 * 2 + 2)
+    {
+    }
+};
+
+constexpr int kRegMaxBorder = 8; // border rows of the register solve: eight lanes take one pair's
+DDCB_HD int reg_border_ints(int k, int nnz) { return (k + 1 + nnz + 1) / 2; }
+DDCB_HD int reg_border_size(SolveTables const& t)
+{
+    return t.k == 0 ? 0 : ((t.cor_lo + t.cor_hi) * t.k * (kRegRows + 1) + t.k * t.k + t.lam_nnz + reg_border_ints(t.k, t.lam_nnz) + 1) / 2 * 2;
+}
 
 // Where the factor entries of row j live in the uploaded tables. Row-major tables (il = 0) store a
 // row's `width` entries together, with the steady run [cj0, cj1) stored once. Interleaved tables
@@ -160,7 +217,7 @@ struct Builder
     double refine_tolerance = 1e-12; // bound on ||A^-1|| |b - A x| / |x| after the last round
     int device = -1;
     int tile_lines = 8;     // lines per CTA
-    int nchunk_req = 64;    // requested chunks per line (64: fastest on 1000-row lines, large and small batches)
+    int nchunk_req = 0;     // requested chunks per line (0: chosen by the plan, HostSolve::make_tables)
     // host copies of the solve tables (for quadrature / transposed host solves)
     int k = 0, m = 0, kl = 0, ku = 0, pivot = 0;
     std::vector<double> lu_band;   // factored Q

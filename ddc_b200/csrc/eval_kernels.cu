@@ -34,10 +34,6 @@ struct EvalArgs
     int lut_smem;       // non-uniform: bucket table copied to shared memory after the knot pairs
 };
 
-__device__ __forceinline__ int64_t line_offset(Lines const& L, int64_t b)
-{
-    return (b / L.inner) * L.outer_stride + (b % L.inner);
-}
 
 __device__ __forceinline__ void cp_async8(void* smem_dst, const void* gmem_src)
 {

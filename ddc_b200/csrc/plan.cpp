@@ -8,6 +8,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <limits>
 #include <cstdio>
 #include <cstdlib>
 #include <map>
@@ -358,6 +359,7 @@ struct HostSolve
     // chunking
     long nchunk = 1, chunk_len = 0, chunk_split = 1, nscan = 0;
     long nscan_f = 0, nscan_b = 0; // scan steps run: later steps' transfers are below 2^-60
+    long ndep_f = 0, ndep_b = 0;   // SolveTables::ndep_f / ndep_b
     std::vector<double> Lf, Uf, PhiF, PhiB;
     std::vector<int8_t> piv;
     long qg_lo = 0, qg_hi = 0;
@@ -579,20 +581,45 @@ struct HostSolve
             chunk_len = 0;
             chunk_split = 1;
         } else {
-            long L = (m + nchunk_req - 1) / std::max<long>(nchunk_req, 1);
-            L = std::max(L, minlen);
-            if (L % 2 == 0) L += 1;
-            nchunk = std::max<long>(1, m / L);
-            chunk_split = nchunk;
-            if (nchunk > 1) {
-                long nc = nchunk, r = m - nc * L;
-                if (r % 2) {
-                    --nc;
-                    r += L;
-                }
-                if (nc > 1 && r / 2 <= nc) {
+            long L = 0;
+            if (nchunk_req <= 0 && m <= kRegMaxChunks * kRegRows && !pivot && kl == ku && kl <= 4) {
+                // as few chunks as keep every chunk within the registers of one thread: long
+                // chunks need fewer carries, and their transfers decay below rounding in a few
+                // chunks. nc chunks of L or L + 2 rows hold m rows when m - nc L is even.
+                for (long nc = (m + kRegRows - 1) / kRegRows; nc <= kRegMaxChunks && L == 0; ++nc) {
+                    long l = std::min<long>(m / nc, kRegRows);
+                    if (l % 2 == 0) --l;
+                    if (l < minlen && nc > 1) break;
+                    long const r = m - nc * l;
+                    if (nc > 1 && (r % 2 || r / 2 > nc || (r > 0 && l + 2 > kRegRows))) continue;
+                    // tiles of eight lines have to fit next to the records (lines of some 1200 to
+                    // 2200 rows, by the band); longer lines are better off with 64 chunks and the
+                    // shared-memory tile
+                    RegRecord const rl {int(kl)};
+                    size_t const bytes = sizeof(double) * size_t(nc * rl.size + 8 * (m + 2 * kl * nc + 8 * k) + 160 * k + k * k);
+                    if (bytes > kRegSmem) break;
                     nchunk = nc;
                     chunk_split = nc - r / 2;
+                    L = l;
+                }
+            }
+            if (L == 0) {
+                long const req = nchunk_req > 0 ? nchunk_req : 64;
+                L = (m + req - 1) / req;
+                L = std::max(L, minlen);
+                if (L % 2 == 0) L += 1;
+                nchunk = std::max<long>(1, m / L);
+                chunk_split = nchunk;
+                if (nchunk > 1) {
+                    long nc = nchunk, r = m - nc * L;
+                    if (r % 2) {
+                        --nc;
+                        r += L;
+                    }
+                    if (nc > 1 && r / 2 <= nc) {
+                        nchunk = nc;
+                        chunk_split = nc - r / 2;
+                    }
                 }
             }
             if (nchunk == 1) {
@@ -663,6 +690,26 @@ struct HostSolve
         };
         nscan_f = kl > 0 ? steps_needed(PhiF, kl) : 0;
         nscan_b = ku > 0 ? steps_needed(PhiB, ku) : 0;
+        // The same bound chunk by chunk: a chunk's incoming carry needs the outgoing carries of the
+        // `t` chunks before it once every product of t transfers is below 2^-60.
+        auto chunks_needed = [&](std::vector<double> const& T, long K, bool fwd) -> long {
+            if (K > 4) return 0; // wide bands: the scan
+            std::vector<double> prod(T), next(T.size());
+            for (long t = 1; t <= kDirectCarry; ++t) {
+                double mx = 0.0;
+                for (double v : prod) mx = std::max(mx, std::fabs(v));
+                if (mx <= 0x1p-60 || t >= nchunk - 1) return t;
+                for (long c = 0; c < nchunk; ++c) {
+                    long const nb = fwd ? c - t : c + t;
+                    if (nb >= 0 && nb < nchunk) matmul(&prod[c * K * K], &T[nb * K * K], &next[c * K * K], K);
+                    else std::fill(&next[c * K * K], &next[c * K * K] + K * K, 0.0);
+                }
+                prod.swap(next);
+            }
+            return 0;
+        };
+        ndep_f = chunks_needed(F, kl, true);
+        ndep_b = chunks_needed(G, ku, false);
     }
 
     // Full host solve of A x = rhs (or A^T x = rhs): used for quadrature coefficients.
@@ -771,6 +818,8 @@ SolveTables upload_tables(HostSolve const& h, std::vector<char>& blob, std::vect
     t.nscan = int(h.nscan);
     t.nscan_f = int(h.nscan_f);
     t.nscan_b = int(h.nscan_b);
+    t.ndep_f = int(h.ndep_f);
+    t.ndep_b = int(h.ndep_b);
     t.lam_nnz = int(h.lam_val.size());
     t.qg_lo = int(h.qg_lo);
     t.qg_hi = int(h.qg_hi);
@@ -876,6 +925,63 @@ SolveTables upload_tables(HostSolve const& h, std::vector<char>& blob, std::vect
     push(arow.data(), arow.size() * 4);
     push(acol.data(), acol.size() * 4);
     push(aval.data(), aval.size() * 8);
+    // the records of the register solve
+    long longest = 0;
+    for (long c = 0; c < h.nchunk && m > 0; ++c) longest = std::max(longest, h.chunk_end(c) - h.chunk_begin(c));
+    t.rmax = (m > 0 && !h.pivot && kl == h.ku && kl <= 4 && longest <= kRegRows && h.nchunk <= kRegMaxChunks
+              && h.ndep_f > 0 && h.ndep_b > 0 && h.k <= kRegMaxBorder)
+                 ? int(longest)
+                 : 0;
+    std::vector<double> rec;
+    if (t.rmax > 0) {
+        RegRecord const L {int(kl)};
+        rec.assign(size_t(h.nchunk) * L.size, 0.0);
+        for (long c = 0; c < h.nchunk; ++c) {
+            double* const r = &rec[size_t(c) * L.size];
+            long const a = h.chunk_begin(c), e = h.chunk_end(c);
+            for (long j = a; j < e; ++j) {
+                std::copy(&h.Lf[j * kl], &h.Lf[j * kl] + kl, r + (j - a) * L.LW);
+                std::copy(&h.Uf[j * ku1], &h.Uf[j * ku1] + ku1, r + L.U + (j - a) * L.UW);
+            }
+            if (h.nscan > 0) { // step 0 of the scan: the chunk's own transfer matrices
+                std::copy(&h.PhiF[c * kl * kl], &h.PhiF[c * kl * kl] + kl * kl, r + L.F);
+                std::copy(&h.PhiB[c * kl * kl], &h.PhiB[c * kl * kl] + kl * kl, r + L.B);
+            }
+        }
+    }
+    push(rec.data(), rec.size() * 8);
+    // the border step of the register solve
+    t.lam_lo = t.lam_hi = t.cor_lo = t.cor_hi = 0;
+    std::vector<double> bord;
+    if (t.rmax > 0 && t.k > 0) {
+        for (int c : h.lam_col) {
+            if (c < m - 1 - c) t.lam_lo = std::max(t.lam_lo, c + 1);
+            else t.lam_hi = std::max(t.lam_hi, int(m) - c);
+        }
+        long const NC = h.nchunk, kk = t.k, W = kRegRows + 1;
+        while (t.cor_lo < NC && h.chunk_begin(t.cor_lo) < h.qg_lo) ++t.cor_lo;
+        while (t.cor_lo + t.cor_hi < NC && h.chunk_end(NC - 1 - t.cor_hi) > m - h.qg_hi) ++t.cor_hi;
+        bord.assign(size_t(reg_border_size(t)), 0.0);
+        double* const g = bord.data();
+        long const nc = t.cor_lo + t.cor_hi;
+        for (long e = 0; e < nc; ++e) {
+            long const c = e < t.cor_lo ? e : NC - nc + e;
+            for (long i = h.chunk_begin(c); i < h.chunk_end(c); ++i) {
+                long const q = i < h.qg_lo ? i : (i >= m - h.qg_hi ? h.qg_lo + i - (m - h.qg_hi) : -1);
+                for (long r = 0; q >= 0 && r < kk; ++r) g[(e * kk + r) * W + i - h.chunk_begin(c)] = h.qg_rows[q * kk + r];
+            }
+        }
+        double* const Si = g + nc * kk * W;
+        std::copy(h.Sinv.begin(), h.Sinv.end(), Si);
+        std::copy(h.lam_val.begin(), h.lam_val.end(), Si + kk * kk);
+        int* const ip = reinterpret_cast<int*>(Si + kk * kk + t.lam_nnz);
+        std::copy(h.lam_row.begin(), h.lam_row.end(), ip);
+        for (long q = 0; q < t.lam_nnz; ++q) {
+            int const c = h.lam_col[q];
+            ip[kk + 1 + q] = c < t.lam_lo ? c : t.lam_lo + c - (int(m) - t.lam_hi);
+        }
+    }
+    push(bord.data(), bord.size() * 8);
     return t;
 }
 
@@ -901,6 +1007,8 @@ void bind_tables(SolveTables& t, char* base, size_t const* offs)
     t.a_row = reinterpret_cast<int const*>(base + offs[17]);
     t.a_col = reinterpret_cast<int const*>(base + offs[18]);
     t.a_val = reinterpret_cast<double const*>(base + offs[19]);
+    t.reg = reinterpret_cast<double const*>(base + offs[20]);
+    t.regb = reinterpret_cast<double const*>(base + offs[21]);
 }
 
 std::string describe(HostSolve const& h)
@@ -1071,7 +1179,7 @@ Builder* create_builder_host(Basis const& basis, double const* pts, long npts, i
         }
         if (b->tile_lines != 2 && b->tile_lines != 4 && b->tile_lines != 8 && b->tile_lines != 16)
             throw Error(DDCB_ERR_INVALID_ARGUMENT, "tile_lines must be 2, 4, 8 or 16");
-        if (b->nchunk_req * b->tile_lines > 1024) throw Error(DDCB_ERR_INVALID_ARGUMENT, "tile_lines*chunks must be <= 1024");
+        if ((b->nchunk_req > 0 ? b->nchunk_req : 64) * b->tile_lines > 1024) throw Error(DDCB_ERR_INVALID_ARGUMENT, "tile_lines*chunks must be <= 1024");
         check_valid_grid(*b);
         // compute_offset (spline_builder.hpp:619-658)
         b->offset = 0;
@@ -1100,6 +1208,9 @@ Builder* create_builder_host(Basis const& basis, double const* pts, long npts, i
             if (top + bottom >= b->n) top = bottom = 0;
         }
         symmetrize_like_reference(rows, *b, top, bottom);
+        auto* priv = new BuilderPrivate();
+        b->host_private = priv;
+        priv->ref_rows = rows;
         b->rrot = int(top);
         b->crot = int(top);
         if (top) {
@@ -1109,10 +1220,6 @@ Builder* create_builder_host(Basis const& basis, double const* pts, long npts, i
                 for (auto const& [j, v] : rows[(i + top) % nn]) rot[i][modulo(j - top, nn)] = v;
             rows.swap(rot);
         }
-        auto* priv = new BuilderPrivate();
-        b->host_private = priv;
-        priv->ref_rows = assemble(*b);
-        symmetrize_like_reference(priv->ref_rows, *b, top, bottom);
         priv->fwd.analyse(rows, D.periodic != 0, top + bottom);
         priv->fwd.make_tables(b->nchunk_req);
         priv->adj.analyse(transpose_rows(rows), D.periodic != 0, top + bottom);
@@ -1314,12 +1421,46 @@ static void emulate_tile_solve(HostSolve const& h, std::vector<double>& T)
     SolveTables tb = upload_tables(h, blob, offs);
     bind_tables(tb, blob.data(), offs.data());
     long const qs = factor_stride(tb);
-    auto Lf_at = [&](long j, long a, long c, long q) { return tb.Lf[factor_base(tb, int(j), int(a), int(c), int(KL)) + q * qs]; };
-    auto Uf_at = [&](long j, long a, long c, long q) { return tb.Uf[factor_base(tb, int(j), int(a), int(c), int(KU + 1)) + q * qs]; };
+    // (the register solve's records hold the same entries)
+    RegRecord const RL {int(std::min(KL, 4L))};
+    auto Lf_at = [&](long j, long a, long c, long q) {
+        double const v = tb.Lf[factor_base(tb, int(j), int(a), int(c), int(KL)) + q * qs];
+        if (tb.rmax == 0) return v;
+        double const r = tb.reg[c * RL.size + (j - a) * RL.LW + q];
+        return r == v ? r : std::numeric_limits<double>::quiet_NaN();
+    };
+    auto Uf_at = [&](long j, long a, long c, long q) {
+        double const v = tb.Uf[factor_base(tb, int(j), int(a), int(c), int(KU + 1)) + q * qs];
+        if (tb.rmax == 0) return v;
+        double const r = tb.reg[c * RL.size + RL.U + (j - a) * RL.UW + q];
+        return r == v ? r : std::numeric_limits<double>::quiet_NaN();
+    };
     auto piv_at = [&](long j, long a, long c) { return long(tb.piv[piv_index(tb, int(j), int(a), int(c))]); };
     std::vector<double> carry(NC * std::max(KL, KU), 0.0), halo(NC * KL, 0.0);
     auto scan = [&](double const* P, long K, bool fwd) {
         std::vector<double> y(carry);
+        long const nd = fwd ? tb.ndep_f : tb.ndep_b;
+        if (nd > 0) { // straight from the outgoing carries of the nd chunks up to c
+            for (long c = 0; c < NC; ++c) {
+                std::vector<double> acc(K, 0.0), v(K);
+                for (long t = nd - 1; t >= 0; --t) {
+                    long const nb = fwd ? c - t : c + t;
+                    if (nb < 0 || nb >= NC) continue;
+                    for (long r = 0; r < K; ++r) {
+                        v[r] = carry[nb * K + r];
+                        for (long q = 0; q < K; ++q) {
+                            double const f = P[scan_index(tb, 0, int(r * K + q), int(nb), int(K))];
+                            bool const same = tb.rmax == 0 || f == tb.reg[nb * RL.size + (fwd ? RL.F : RL.B) + r * K + q];
+                            v[r] += (same ? f : std::numeric_limits<double>::quiet_NaN()) * acc[q];
+                        }
+                    }
+                    acc = v;
+                }
+                std::copy(acc.begin(), acc.end(), &y[c * K]);
+            }
+            carry = y;
+            return;
+        }
         for (long s = 0; s < (fwd ? tb.nscan_f : tb.nscan_b); ++s) {
             std::vector<double> next(y);
             for (long c = 0; c < NC; ++c) {
@@ -1343,7 +1484,7 @@ static void emulate_tile_solve(HostSolve const& h, std::vector<double>& T)
             std::vector<double> w(KL + 1, 0.0);
             for (long q = 0; q < KL; ++q) w[q] = (a + q < m) ? T[a + q] : 0.0;
             for (long j = a; j < e; ++j) {
-                w[KL] = (j + KL < m) ? T[j + KL] : 0.0;
+                w[KL] = (j + KL < (h.pivot ? m : e)) ? T[j + KL] : 0.0;
                 long const p = piv_at(j, a, c);
                 if (p) std::swap(w[0], w[p]);
                 double const y = w[0];
@@ -1352,7 +1493,7 @@ static void emulate_tile_solve(HostSolve const& h, std::vector<double>& T)
             }
             for (long q = 0; q < KL; ++q) {
                 double const orig = (e + q < m) ? T[e + q] : 0.0;
-                carry[c * KL + q] = w[q] - orig;
+                carry[c * KL + q] = h.pivot ? w[q] - orig : w[q];
                 halo[c * KL + q] = orig;
             }
         }
@@ -1381,7 +1522,7 @@ static void emulate_tile_solve(HostSolve const& h, std::vector<double>& T)
             std::vector<double> z(KU, 0.0);
             for (long j = e - 1; j >= a; --j) {
                 double s = T[j];
-                for (long q = 1; q <= KU; ++q) s -= Uf_at(j, a, c, q) * z[q - 1];
+                for (long q = KU; q >= 1; --q) s -= Uf_at(j, a, c, q) * z[q - 1];
                 double const x = s * Uf_at(j, a, c, 0);
                 for (long q = KU - 1; q >= 1; --q) z[q] = z[q - 1];
                 z[0] = x;
@@ -1395,7 +1536,7 @@ static void emulate_tile_solve(HostSolve const& h, std::vector<double>& T)
             for (long q = 0; q < KU; ++q) z[q] = (c + 1 < NC) ? carry[(c + 1) * KU + q] : 0.0;
             for (long j = e - 1; j >= a; --j) {
                 double s = T[j];
-                for (long q = 1; q <= KU; ++q) s -= Uf_at(j, a, c, q) * z[q - 1];
+                for (long q = KU; q >= 1; --q) s -= Uf_at(j, a, c, q) * z[q - 1];
                 double const x = s * Uf_at(j, a, c, 0);
                 Tn[j] = x;
                 for (long q = KU - 1; q >= 1; --q) z[q] = z[q - 1];
@@ -1409,6 +1550,30 @@ static void emulate_tile_solve(HostSolve const& h, std::vector<double>& T)
         for (long r = 0; r < k; ++r) bt[r] = T[m + r];
         for (long r = 0; r < k; ++r)
             for (int q = h.lam_row[r]; q < h.lam_row[r + 1]; ++q) bt[r] -= h.lam_val[q] * T[h.lam_col[q]];
+        // the register solve's border block holds the same numbers
+        if (tb.rmax > 0) {
+            long const nc = tb.cor_lo + tb.cor_hi, W = kRegRows + 1;
+            double const* Si = tb.regb + nc * k * W;
+            int const* ip = reinterpret_cast<int const*>(Si + k * k + tb.lam_nnz);
+            bool same = true;
+            for (long r = 0; r <= k; ++r) same = same && ip[r] == h.lam_row[r];
+            for (long q = 0; q < tb.lam_nnz; ++q) {
+                long const e = ip[k + 1 + q];
+                same = same && (e < tb.lam_lo ? e : m - tb.lam_hi + (e - tb.lam_lo)) == h.lam_col[q] && Si[k * k + q] == h.lam_val[q];
+            }
+            for (long q = 0; q < k * k; ++q) same = same && Si[q] == h.Sinv[q];
+            long corrected = 0;
+            for (long e = 0; e < nc; ++e) {
+                long const c = e < tb.cor_lo ? e : NC - nc + e;
+                for (long i = h.chunk_begin(c); i < h.chunk_end(c); ++i) {
+                    long const q = i < h.qg_lo ? i : (i >= m - h.qg_hi ? h.qg_lo + i - (m - h.qg_hi) : -1);
+                    corrected += q >= 0;
+                    for (long r = 0; r < k; ++r)
+                        same = same && tb.regb[(e * k + r) * W + i - h.chunk_begin(c)] == (q >= 0 ? h.qg_rows[q * k + r] : 0.0);
+                }
+            }
+            if (!same || corrected != h.qg_lo + h.qg_hi) bt.assign(k, std::numeric_limits<double>::quiet_NaN());
+        }
         for (long r = 0; r < k; ++r) {
             double s = 0.0;
             for (long q = 0; q < k; ++q) s += h.Sinv[r * k + q] * bt[q];
