@@ -230,25 +230,53 @@ namespace ddcb {
 
 // ---- compile-time-degree device forms used by the kernels ------------------------------------
 
-// Uniform Cox-de Boor values of degree P from the cell offset; the divisions by the small integer
-// j are multiplications by its rounded reciprocal.
+// Uniform Cox-de Boor values of degree P from the cell offset, times P!: the levels' divisions by
+// j = 1 .. P are left to one factor at the end (factorial_inverse), and the distances to the knots
+// are formed once. 15 operations for a cubic instead of 28.
+template <int P>
+DDCB_HD void uniform_values_raw(double offset, double* v)
+{
+    double below[P + 1], above[P + 1]; // offset + k and k - offset: distances to knots either side
+    below[0] = offset;
+#pragma unroll
+    for (int k = 1; k <= P; ++k) {
+        below[k] = offset + k;
+        above[k] = k - offset;
+    }
+    v[0] = 1.0;
+    if (P > 0) {
+        v[0] = above[1];
+        v[1] = offset;
+    }
+#pragma unroll
+    for (int j = 2; j <= P; ++j) {
+        double saved = below[j - 1] * v[0];
+        v[0] = above[1] * v[0];
+#pragma unroll
+        for (int r = 1; r < j; ++r) {
+            double const t = v[r];
+            v[r] = saved + above[r + 1] * t;
+            saved = below[j - 1 - r] * t;
+        }
+        v[j] = saved;
+    }
+}
+
+DDCB_HD constexpr double factorial_inverse(int p)
+{
+    double f = 1.0;
+    for (int j = 2; j <= p; ++j) f *= j;
+    return 1.0 / f;
+}
+
+// The values themselves.
 template <int P>
 DDCB_HD void uniform_values_t(double offset, double* v)
 {
-    v[0] = 1.0;
+    uniform_values_raw<P>(offset, v);
+    if (P > 1) {
 #pragma unroll
-    for (int j = 1; j <= P; ++j) {
-        double const inv_j = 1.0 / j;
-        double xx = -offset;
-        double saved = 0.0;
-#pragma unroll
-        for (int r = 0; r < j; ++r) {
-            xx += 1.0;
-            double const temp = v[r] * inv_j;
-            v[r] = saved + xx * temp;
-            saved = (j - xx) * temp;
-        }
-        v[j] = saved;
+        for (int r = 0; r <= P; ++r) v[r] *= factorial_inverse(P);
     }
 }
 

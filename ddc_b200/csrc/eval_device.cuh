@@ -319,7 +319,7 @@ __device__ __forceinline__ double eval_value_no_bc(EvalBasis const& eb, double x
     if (UNI) {
         double off;
         jmin = uniform_cell(eb.b, x, off);
-        uniform_values_t<D>(off, v);
+        uniform_values_raw<D>(off, v);
     } else {
         double kn[2 * D];
         jmin = locate_load_knots<D>(eb, x, kn) - D;
@@ -329,7 +329,7 @@ __device__ __forceinline__ double eval_value_no_bc(EvalBasis const& eb, double x
     double y = 0.0;
 #pragma unroll
     for (int i = 0; i < D + 1; ++i) y = fma(C.get(r0, i), v[i], y);
-    return y;
+    return UNI && D > 1 ? y * factorial_inverse(D) : y;
 }
 
 // s(x) with the periodic wrap or the extrapolation rules (spline_evaluator.hpp:529-554,
@@ -368,7 +368,7 @@ __device__ __forceinline__ double eval_deriv_no_bc(EvalBasis const& eb, double x
     if (UNI) {
         double off;
         jmin = uniform_cell(eb.b, x, off);
-        uniform_values_t<P>(off, v);
+        uniform_values_raw<P>(off, v);
     } else {
         int const ck = nonuniform_locate(eb, x);
         jmin = ck - D;
@@ -395,7 +395,7 @@ __device__ __forceinline__ double eval_deriv_no_bc(EvalBasis const& eb, double x
     double y = 0.0;
 #pragma unroll
     for (int r = 0; r < P + 1; ++r) y = fma(cc[ORDER + r], v[r], y);
-    return y;
+    return UNI && P > 1 ? y * factorial_inverse(P) : y;
 }
 
 // Value (ORDER 0, with boundary handling) or ORDER-th derivative (no boundary handling).
@@ -469,6 +469,26 @@ __device__ __forceinline__ int basis_derivs(EvalBasis const& eb, double x, doubl
 #pragma unroll
     for (int i = 0; i <= D; ++i) val[i] = w[i];
     return jmin;
+}
+
+// basis_derivs up to the factor basis_scale: uniform values keep their level divisions for one
+// multiplication of the finished sum.
+template <int D, int ORDER, bool UNI>
+__device__ __forceinline__ int basis_raw(EvalBasis const& eb, double x, double* val)
+{
+    if constexpr (UNI && ORDER == 0) {
+        double off;
+        int const jmin = uniform_cell(eb.b, x, off);
+        uniform_values_raw<D>(off, val);
+        return jmin;
+    } else {
+        return basis_derivs<D, ORDER, UNI>(eb, x, val);
+    }
+}
+template <int D, int ORDER, bool UNI>
+__device__ constexpr double basis_scale()
+{
+    return UNI && ORDER == 0 ? factorial_inverse(D) : 1.0;
 }
 
 // Reverse mode of one evaluated point. For y = s(x) (ORDER 0, with the boundary handling of

@@ -6,9 +6,8 @@
 // x2 pass over the result), run by the 1D build kernel with strided line descriptors. The batch is
 // processed in groups of fields whose x1-pass result fits comfortably in L2, so the x2 pass reads
 // it back from L2 rather than HBM; the workspace holds one group.
-// Evaluator: a warp handles 32 fields of one point, so each of the (d1+1)(d2+1) coefficient
-// gathers is one coalesced 256-byte load, and consecutive points of a block share coefficients
-// through L1.
+// Evaluator: neighbouring lanes take neighbouring fields of one point, so the (d1+1)(d2+1) coefficient
+// gathers are coalesced, and consecutive points of a block share coefficients through L1.
 #include <algorithm>
 #include <mutex>
 #include <string>
@@ -134,31 +133,11 @@ struct Eval2dArgs
     int64_t m, B, size2;
 };
 
-template <int D1, int D2, int O1, int O2, bool U1, bool U2>
-__device__ __forceinline__ double eval2d_point(Eval2dArgs const& a, double x1, double x2, const double* C)
-{
-    double v1[D1 + 1], v2[D2 + 1];
-    int const j1 = basis_derivs<D1, O1, U1>(a.e1, x1, v1);
-    int const j2 = basis_derivs<D2, O2, U2>(a.e2, x2, v2);
-    int64_t const B = a.B;
-    double y = 0.0;
-#pragma unroll
-    for (int i = 0; i < D1 + 1; ++i) {
-        const double* row = C + ((int64_t)(j1 + i) * a.size2 + j2) * B;
-        double t = 0.0;
-#pragma unroll
-        for (int j = 0; j < D2 + 1; ++j) t = fma(__ldg(row + j * B), v2[j], t);
-        y = fma(t, v1[i], y);
-    }
-    return y;
-}
-
 // Boundary handling of SplineEvaluator2D::eval (spline_evaluator_2d.hpp:680-727): periodic wraps,
-// then the extrapolation rules of the non-periodic dimensions (null: 0; constant: the value at the
-// domain end, the other coordinate clamped when that dimension is not periodic,
+// then the extrapolation rules of the non-periodic dimensions (null: 0, returned as false; constant:
+// the value at the domain end, the other coordinate clamped when that dimension is not periodic,
 // constant_extrapolation_rule.hpp:143-193).
-template <int D1, int D2, bool U1, bool U2>
-__device__ __forceinline__ double eval2d_bc(Eval2dArgs const& a, double x1, double x2, const double* C)
+__device__ __forceinline__ bool place2d(Eval2dArgs const& a, double& x1, double& x2)
 {
     BasisDesc const& b1 = a.e1.b;
     BasisDesc const& b2 = a.e2.b;
@@ -167,50 +146,108 @@ __device__ __forceinline__ double eval2d_bc(Eval2dArgs const& a, double x1, doub
     auto clamp = [](double v, double lo, double hi) { return v < lo ? lo : (v > hi ? hi : v); };
     if (!b1.periodic && (x1 < b1.rmin || x1 > b1.rmax)) {
         bool const low = x1 < b1.rmin;
-        if ((low ? a.ex1lo : a.ex1hi) == 1) return 0.0;
+        if ((low ? a.ex1lo : a.ex1hi) == 1) return false;
         x1 = low ? b1.rmin : b1.rmax;
         if (!b2.periodic) x2 = clamp(x2, b2.rmin, b2.rmax);
     } else if (!b2.periodic && (x2 < b2.rmin || x2 > b2.rmax)) {
         bool const low = x2 < b2.rmin;
-        if ((low ? a.ex2lo : a.ex2hi) == 1) return 0.0;
+        if ((low ? a.ex2lo : a.ex2hi) == 1) return false;
         x2 = low ? b2.rmin : b2.rmax;
         if (!b1.periodic) x1 = clamp(x1, b1.rmin, b1.rmax);
     }
-    return eval2d_point<D1, D2, 0, 0, U1, U2>(a, x1, x2, C);
+    return true;
 }
 
-constexpr int kPts2d = 8; // points (warps) per block; 32 fields per warp
+// A point of one field (V = double) or of two neighbouring fields that share it (double2).
+// C: the fields' coefficients.
+template <int D1, int D2, int O1, int O2, bool U1, bool U2, class V>
+__device__ __forceinline__ V eval2d_point(Eval2dArgs const& a, double x1, double x2, const double* C)
+{
+    V y = zero_of<V>();
+    if (O1 == 0 && O2 == 0 && !place2d(a, x1, x2)) return y;
+    double v1[D1 + 1], v2[D2 + 1];
+    int const j1 = basis_raw<D1, O1, U1>(a.e1, x1, v1);
+    int const j2 = basis_raw<D2, O2, U2>(a.e2, x2, v2);
+    int64_t const B = a.B;
+    const double* row = C + ((int64_t)j1 * a.size2 + j2) * B;
+#pragma unroll
+    for (int i = 0; i < D1 + 1; ++i) {
+        V t = zero_of<V>();
+        const double* c = row;
+#pragma unroll
+        for (int j = 0; j < D2 + 1; ++j) {
+            t = fma2(v2[j], __ldg(reinterpret_cast<const V*>(c)), t);
+            c += B;
+        }
+        y = fma2(v1[i], t, y);
+        row += a.size2 * B;
+    }
+    constexpr double scale = basis_scale<D1, O1, U1>() * basis_scale<D2, O2, U2>();
+    return scale == 1.0 ? y : mul2(y, scale);
+}
+
+constexpr int kThreads2d = 256;
+constexpr int kItems2d = 2048; // (point, field) items per block, over at most 32 columns
+
+// A block evaluates ppb consecutive points for hs of the H columns of fields: single fields, or
+// (PAIR) pairs of neighbouring fields, which share basis and position and load their coefficients as
+// 16-byte vectors where their points coincide (feet computed once for all fields), else take turns.
+// Items are numbered point by point, so few fields fill a warp with several points.
+template <int D1, int D2, int O1, int O2, bool U1, bool U2, bool PAIR>
+__global__ void __launch_bounds__(kThreads2d) eval2d_kernel(const __grid_constant__ Eval2dArgs a, int ppb, int H, int hs)
+{
+    int const h0 = blockIdx.y * hs;
+    hs = min(hs, H - h0);
+    int64_t const p0 = (int64_t)blockIdx.x * ppb;
+    int const np = int(min((int64_t)ppb, a.m - p0));
+    int q = threadIdx.x / hs, h = threadIdx.x - q * hs;
+    int const dq = kThreads2d / hs, dh = kThreads2d - dq * hs;
+    while (q < np) {
+        int64_t const at = (p0 + q) * a.B + (PAIR ? 2 : 1) * (h0 + h);
+        const double* const C = a.coefs + (PAIR ? 2 : 1) * (h0 + h);
+        const double2* const xy = reinterpret_cast<const double2*>(a.coords) + at;
+        double2 const u = __ldcs(xy);
+        if constexpr (PAIR) {
+            double2 const w = __ldcs(xy + 1);
+            double2 y;
+            if (u.x == w.x && u.y == w.y) {
+                y = eval2d_point<D1, D2, O1, O2, U1, U2, double2>(a, u.x, u.y, C);
+            } else {
+                y.x = eval2d_point<D1, D2, O1, O2, U1, U2, double>(a, u.x, u.y, C);
+                y.y = eval2d_point<D1, D2, O1, O2, U1, U2, double>(a, w.x, w.y, C + 1);
+            }
+            __stcs(reinterpret_cast<double2*>(a.out + at), y);
+        } else {
+            __stcs(a.out + at, eval2d_point<D1, D2, O1, O2, U1, U2, double>(a, u.x, u.y, C));
+        }
+        q += dq;
+        h += dh;
+        if (h >= hs) {
+            h -= hs;
+            ++q;
+        }
+    }
+}
 
 template <int D1, int D2, int O1, int O2, bool U1, bool U2>
-__global__ void __launch_bounds__(32 * kPts2d) eval2d_kernel(const __grid_constant__ Eval2dArgs a, int64_t pts_per_block)
+void launch_eval2d_p(Eval2dArgs const& a, cudaStream_t s)
 {
-    int const lane = threadIdx.x & 31;
-    int const w = threadIdx.x >> 5;
-    int64_t const b = (int64_t)blockIdx.y * 32 + lane;
-    if (b >= a.B) return;
-    int64_t const p0 = (int64_t)blockIdx.x * pts_per_block;
-    int64_t const p1 = min(p0 + pts_per_block, a.m);
-    const double* C = a.coefs + b;
-    for (int64_t p = p0 + w; p < p1; p += kPts2d) {
-        double2 const xy = reinterpret_cast<const double2*>(a.coords)[p * a.B + b];
-        double y;
-        if (O1 == 0 && O2 == 0) y = eval2d_bc<D1, D2, U1, U2>(a, xy.x, xy.y, C);
-        else y = eval2d_point<D1, D2, O1, O2, U1, U2>(a, xy.x, xy.y, C);
-        a.out[p * a.B + b] = y;
-    }
+    bool const pair = a.B % 2 == 0 && reinterpret_cast<uintptr_t>(a.coefs) % 16 == 0 && reinterpret_cast<uintptr_t>(a.out) % 16 == 0;
+    int const H = int(pair ? a.B / 2 : a.B), hs = std::min(H, 32), ppb = kItems2d / hs;
+    dim3 const grid((unsigned)((a.m + ppb - 1) / ppb), (unsigned)((H + hs - 1) / hs));
+    if (pair) eval2d_kernel<D1, D2, O1, O2, U1, U2, true><<<grid, kThreads2d, 0, s>>>(a, ppb, H, hs);
+    else eval2d_kernel<D1, D2, O1, O2, U1, U2, false><<<grid, kThreads2d, 0, s>>>(a, ppb, H, hs);
+    DDCB_CUDA_CHECK(cudaGetLastError());
 }
 
 template <int D1, int D2, int O1, int O2>
 void launch_eval2d_u(Eval2dArgs const& a, cudaStream_t s)
 {
-    int64_t const ppb = 64;
-    dim3 grid((unsigned)((a.m + ppb - 1) / ppb), (unsigned)((a.B + 31) / 32));
     bool const u1 = a.e1.b.uniform != 0, u2 = a.e2.b.uniform != 0;
-    if (u1 && u2) eval2d_kernel<D1, D2, O1, O2, true, true><<<grid, 32 * kPts2d, 0, s>>>(a, ppb);
-    else if (u1) eval2d_kernel<D1, D2, O1, O2, true, false><<<grid, 32 * kPts2d, 0, s>>>(a, ppb);
-    else if (u2) eval2d_kernel<D1, D2, O1, O2, false, true><<<grid, 32 * kPts2d, 0, s>>>(a, ppb);
-    else eval2d_kernel<D1, D2, O1, O2, false, false><<<grid, 32 * kPts2d, 0, s>>>(a, ppb);
-    DDCB_CUDA_CHECK(cudaGetLastError());
+    if (u1 && u2) launch_eval2d_p<D1, D2, O1, O2, true, true>(a, s);
+    else if (u1) launch_eval2d_p<D1, D2, O1, O2, true, false>(a, s);
+    else if (u2) launch_eval2d_p<D1, D2, O1, O2, false, true>(a, s);
+    else launch_eval2d_p<D1, D2, O1, O2, false, false>(a, s);
 }
 
 template <int D1, int D2>

@@ -15,10 +15,10 @@
 // the values, then the 2D builder over dimensions 2-3) with the intermediate arrays of one
 // layout, so passes 2 and 3 are a single launch each.
 //
-// Evaluator. A warp evaluates one point of 32 batch entries: each lane computes the basis of its
-// own coordinates dimension by dimension (degree and derivative order chosen at run time), and the
-// prod(d_k + 1) coefficient gathers of a point are coalesced 256-byte loads when the lanes share
-// the point's cell. Values of 3D splines with one degree in all dimensions run an unrolled kernel
+// Evaluator. Neighbouring lanes take neighbouring batch entries of one point: each lane computes the
+// basis of its own coordinates dimension by dimension (degree and derivative order chosen at run
+// time), and the prod(d_k + 1) coefficient gathers of a point are coalesced when the lanes share the
+// point's cell. Values of 3D splines with one degree in all dimensions run an unrolled kernel
 // (the basis in registers, the (d+1)^3 gathers unrolled); other cases the general one.
 #include <algorithm>
 #include <string>
@@ -129,7 +129,8 @@ void launch_build3d(Builder const& b1, Builder const& b2, Builder const& b3, dou
 // ---------------------------------------------------------------------------------------------
 namespace {
 
-constexpr int kPtsNd = 8; // points (warps) per block; 32 batch entries per warp
+constexpr int kThreadsNd = 256;
+constexpr int kItemsNd = 2048; // (point, batch entry) items per block, over at most 32 columns
 
 struct EvalNdArgs
 {
@@ -199,17 +200,33 @@ __device__ double tensor_sum(EvalNdArgs const& a, const double* C, const int* jm
     return y;
 }
 
-__global__ void __launch_bounds__(32 * kPtsNd) evalnd_kernel(const __grid_constant__ EvalNdArgs a, int64_t pts_per_block)
+// The (point, column) items of a block: ppb consecutive points, hs of the H columns, numbered point by
+// point, so that few batch entries fill a warp with several points. f(point, column).
+template <class F>
+__device__ __forceinline__ void for_items(int64_t m, int ppb, int H, int hs, F f)
 {
-    int const lane = threadIdx.x & 31;
-    int const wp = threadIdx.x >> 5;
-    int64_t const b = (int64_t)blockIdx.y * 32 + lane;
-    if (b >= a.B) return;
-    int64_t const p0 = (int64_t)blockIdx.x * pts_per_block;
-    int64_t const p1 = min(p0 + pts_per_block, a.m);
+    int const h0 = blockIdx.y * hs;
+    hs = min(hs, H - h0);
+    int64_t const p0 = (int64_t)blockIdx.x * ppb;
+    int const np = int(min((int64_t)ppb, m - p0));
+    int q = threadIdx.x / hs, h = threadIdx.x - q * hs;
+    int const dq = kThreadsNd / hs, dh = kThreadsNd - dq * hs;
+    while (q < np) {
+        f(p0 + q, h0 + h);
+        q += dq;
+        h += dh;
+        if (h >= hs) {
+            h -= hs;
+            ++q;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kThreadsNd) evalnd_kernel(const __grid_constant__ EvalNdArgs a, int ppb, int H, int hs)
+{
     int const N = a.ndims;
-    const double* C = a.coefs + b;
-    for (int64_t p = p0 + wp; p < p1; p += kPtsNd) {
+    for_items(a.m, ppb, H, hs, [&](int64_t p, int b) {
+        const double* C = a.coefs + b;
         const double* xp = a.coords + (p * a.B + b) * N;
         double x[kMaxDims];
         for (int d = 0; d < N; ++d) x[d] = xp[d];
@@ -246,74 +263,114 @@ __global__ void __launch_bounds__(32 * kPtsNd) evalnd_kernel(const __grid_consta
             y = tensor_sum(a, C, jmin, v);
         }
         a.out[p * a.B + b] = y;
-    }
+    });
 }
 
 // Values (with the boundary handling of evalnd_kernel) of a 3D spline whose three dimensions share
 // one degree D: the basis of each dimension in registers and the (D+1)^3 gathers unrolled.
-template <int D>
-__device__ __forceinline__ int basis_values_any(EvalBasis const& eb, double x, double* v)
+// place3d: periodic wraps and extrapolation rules; false where the value is 0.
+__device__ __forceinline__ bool place3d(EvalNdArgs const& a, double* x)
 {
-    return eb.b.uniform ? basis_derivs<D, 0, true>(eb, x, v) : basis_derivs<D, 0, false>(eb, x, v);
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+        if (a.eb[d].b.periodic) x[d] = periodic_wrap(a.eb[d].b, x[d]);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        BasisDesc const& bd = a.eb[d].b;
+        if (bd.periodic || (x[d] >= bd.rmin && x[d] <= bd.rmax)) continue;
+        bool const low = x[d] < bd.rmin;
+        if ((low ? a.ex_lo[d] : a.ex_hi[d]) == DDCB_EXTRAP_NULL) return false;
+        x[d] = low ? bd.rmin : bd.rmax;
+#pragma unroll
+        for (int e = 0; e < 3; ++e) {
+            BasisDesc const& be = a.eb[e].b;
+            if (e != d && !be.periodic) x[e] = x[e] < be.rmin ? be.rmin : (x[e] > be.rmax ? be.rmax : x[e]);
+        }
+        break;
+    }
+    return true;
+}
+
+// Basis values of one dimension up to `scale`, which is multiplied into.
+template <int D>
+__device__ __forceinline__ int basis_values_any(EvalBasis const& eb, double x, double* v, double& scale)
+{
+    if (eb.b.uniform) {
+        scale *= basis_scale<D, 0, true>();
+        return basis_raw<D, 0, true>(eb, x, v);
+    }
+    return basis_derivs<D, 0, false>(eb, x, v);
+}
+
+// A point of one batch entry (V = double) or of two neighbouring ones that share it (double2).
+template <int D, class V>
+__device__ __forceinline__ V eval3d_point(EvalNdArgs const& a, double x0, double x1, double x2, const double* C)
+{
+    double x[3] = {x0, x1, x2};
+    V y = zero_of<V>();
+    if (!place3d(a, x)) return y;
+    double v0[D + 1], v1[D + 1], v2[D + 1];
+    double scale = 1.0;
+    int const j0 = DDCB_INDEX(basis_values_any<D>(a.eb[0], x[0], v0, scale), a.eb[0].b.ncells);
+    int const j1 = DDCB_INDEX(basis_values_any<D>(a.eb[1], x[1], v1, scale), a.eb[1].b.ncells);
+    int const j2 = DDCB_INDEX(basis_values_any<D>(a.eb[2], x[2], v2, scale), a.eb[2].b.ncells);
+    const double* plane = C + (int64_t)j0 * a.cstride[0] + (int64_t)j1 * a.cstride[1] + (int64_t)j2 * a.cstride[2];
+#pragma unroll
+    for (int i0 = 0; i0 <= D; ++i0) {
+        V t1 = zero_of<V>();
+        const double* row = plane;
+#pragma unroll
+        for (int i1 = 0; i1 <= D; ++i1) {
+            V t2 = zero_of<V>();
+            const double* c = row;
+#pragma unroll
+            for (int i2 = 0; i2 <= D; ++i2) {
+                t2 = fma2(v2[i2], __ldg(reinterpret_cast<const V*>(c)), t2);
+                c += a.cstride[2];
+            }
+            t1 = fma2(v1[i1], t2, t1);
+            row += a.cstride[1];
+        }
+        y = fma2(v0[i0], t1, y);
+        plane += a.cstride[0];
+    }
+    return mul2(y, scale);
+}
+
+// Columns are batch entries, or (PAIR) pairs of neighbouring ones, which share the basis and load
+// their coefficients as 16-byte vectors where their points coincide, and take turns where not.
+template <int D, bool PAIR>
+__global__ void __launch_bounds__(kThreadsNd) eval3d_kernel(const __grid_constant__ EvalNdArgs a, int ppb, int H, int hs)
+{
+    for_items(a.m, ppb, H, hs, [&](int64_t p, int h) {
+        int64_t const at = p * a.B + (PAIR ? 2 * h : h);
+        const double* const C = a.coefs + (PAIR ? 2 * h : h);
+        const double* const x = a.coords + at * 3;
+        double const x0 = __ldcs(x), x1 = __ldcs(x + 1), x2 = __ldcs(x + 2);
+        if constexpr (PAIR) {
+            double const u0 = __ldcs(x + 3), u1 = __ldcs(x + 4), u2 = __ldcs(x + 5);
+            double2 y;
+            if (x0 == u0 && x1 == u1 && x2 == u2) {
+                y = eval3d_point<D, double2>(a, x0, x1, x2, C);
+            } else {
+                y.x = eval3d_point<D, double>(a, x0, x1, x2, C);
+                y.y = eval3d_point<D, double>(a, u0, u1, u2, C + 1);
+            }
+            __stcs(reinterpret_cast<double2*>(a.out + at), y);
+        } else {
+            __stcs(a.out + at, eval3d_point<D, double>(a, x0, x1, x2, C));
+        }
+    });
 }
 
 template <int D>
-__global__ void __launch_bounds__(32 * kPtsNd) eval3d_kernel(const __grid_constant__ EvalNdArgs a, int64_t pts_per_block)
+void launch_eval3d(EvalNdArgs const& a, cudaStream_t s)
 {
-    int const lane = threadIdx.x & 31;
-    int const wp = threadIdx.x >> 5;
-    int64_t const b = (int64_t)blockIdx.y * 32 + lane;
-    if (b >= a.B) return;
-    int64_t const p0 = (int64_t)blockIdx.x * pts_per_block;
-    int64_t const p1 = min(p0 + pts_per_block, a.m);
-    const double* C = a.coefs + b;
-    for (int64_t p = p0 + wp; p < p1; p += kPtsNd) {
-        const double* xp = a.coords + (p * a.B + b) * 3;
-        double x[3] = {xp[0], xp[1], xp[2]};
-        double y = 0.0;
-        bool zero = false;
-#pragma unroll
-        for (int d = 0; d < 3; ++d)
-            if (a.eb[d].b.periodic) x[d] = periodic_wrap(a.eb[d].b, x[d]);
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            BasisDesc const& bd = a.eb[d].b;
-            if (zero || bd.periodic || (x[d] >= bd.rmin && x[d] <= bd.rmax)) continue;
-            bool const low = x[d] < bd.rmin;
-            if ((low ? a.ex_lo[d] : a.ex_hi[d]) == DDCB_EXTRAP_NULL) {
-                zero = true;
-            } else {
-                x[d] = low ? bd.rmin : bd.rmax;
-#pragma unroll
-                for (int e = 0; e < 3; ++e) {
-                    BasisDesc const& be = a.eb[e].b;
-                    if (e != d && !be.periodic) x[e] = x[e] < be.rmin ? be.rmin : (x[e] > be.rmax ? be.rmax : x[e]);
-                }
-                break;
-            }
-        }
-        if (!zero) {
-            double v0[D + 1], v1[D + 1], v2[D + 1];
-            int const j0 = DDCB_INDEX(basis_values_any<D>(a.eb[0], x[0], v0), a.eb[0].b.ncells);
-            int const j1 = DDCB_INDEX(basis_values_any<D>(a.eb[1], x[1], v1), a.eb[1].b.ncells);
-            int const j2 = DDCB_INDEX(basis_values_any<D>(a.eb[2], x[2], v2), a.eb[2].b.ncells);
-#pragma unroll
-            for (int i0 = 0; i0 <= D; ++i0) {
-                double t1 = 0.0;
-#pragma unroll
-                for (int i1 = 0; i1 <= D; ++i1) {
-                    const double* row = C + (int64_t)(j0 + i0) * a.cstride[0] + (int64_t)(j1 + i1) * a.cstride[1]
-                                        + (int64_t)j2 * a.cstride[2];
-                    double t2 = 0.0;
-#pragma unroll
-                    for (int i2 = 0; i2 <= D; ++i2) t2 = fma(__ldg(row + i2 * a.cstride[2]), v2[i2], t2);
-                    t1 = fma(t2, v1[i1], t1);
-                }
-                y = fma(t1, v0[i0], y);
-            }
-        }
-        a.out[p * a.B + b] = y;
-    }
+    bool const pair = a.B % 2 == 0 && reinterpret_cast<uintptr_t>(a.coefs) % 16 == 0 && reinterpret_cast<uintptr_t>(a.out) % 16 == 0;
+    int const H = int(pair ? a.B / 2 : a.B), hs = std::min(H, 32), ppb = kItemsNd / hs;
+    dim3 const grid((unsigned)((a.m + ppb - 1) / ppb), (unsigned)((H + hs - 1) / hs));
+    if (pair) eval3d_kernel<D, true><<<grid, kThreadsNd, 0, s>>>(a, ppb, H, hs);
+    else eval3d_kernel<D, false><<<grid, kThreadsNd, 0, s>>>(a, ppb, H, hs);
 }
 
 struct IntegrateNdArgs
@@ -379,21 +436,21 @@ void launch_evalnd(Evaluator const* const* e, int ndims, int const* orders, doub
     a.out = out;
     a.m = m;
     a.B = B;
-    int64_t const ppb = 64;
-    dim3 grid((unsigned)((m + ppb - 1) / ppb), (unsigned)((B + 31) / 32));
     // 3D values with one degree in every dimension: the unrolled kernel
     int const D0 = e[0]->basis.desc.degree;
     bool const same3 = ndims == 3 && orders == nullptr && e[1]->basis.desc.degree == D0 && e[2]->basis.desc.degree == D0;
     if (same3) {
         switch (D0) {
-        case 1: eval3d_kernel<1><<<grid, 32 * kPtsNd, 0, s>>>(a, ppb); break;
-        case 2: eval3d_kernel<2><<<grid, 32 * kPtsNd, 0, s>>>(a, ppb); break;
-        case 3: eval3d_kernel<3><<<grid, 32 * kPtsNd, 0, s>>>(a, ppb); break;
-        case 4: eval3d_kernel<4><<<grid, 32 * kPtsNd, 0, s>>>(a, ppb); break;
-        default: eval3d_kernel<5><<<grid, 32 * kPtsNd, 0, s>>>(a, ppb); break;
+        case 1: launch_eval3d<1>(a, s); break;
+        case 2: launch_eval3d<2>(a, s); break;
+        case 3: launch_eval3d<3>(a, s); break;
+        case 4: launch_eval3d<4>(a, s); break;
+        default: launch_eval3d<5>(a, s); break;
         }
     } else {
-        evalnd_kernel<<<grid, 32 * kPtsNd, 0, s>>>(a, ppb);
+        int const hs = int(std::min<int64_t>(B, 32)), ppb = kItemsNd / hs;
+        dim3 const grid((unsigned)((m + ppb - 1) / ppb), (unsigned)((B + hs - 1) / hs));
+        evalnd_kernel<<<grid, kThreadsNd, 0, s>>>(a, ppb, int(B), hs);
     }
     DDCB_CUDA_CHECK(cudaGetLastError());
 }
