@@ -8,27 +8,11 @@
 // exist for the band shapes and tile width the configurations use; any other combination runs the
 // builder and the evaluator kernels one after the other (same results).
 #include "build_device.cuh"
-#include "eval_device.cuh"
+#include "fused_eval.hpp"
 
 namespace ddcb {
 
 namespace {
-
-struct FusedEval
-{
-    EvalBasis eb;
-    int ex_lo, ex_hi;
-    const double* coords;
-    Lines lx;
-    double* out;
-    Lines lo;
-    // FEET kernels (the advection step): point q of line b is at pts[q] - dt * v(b), with
-    // v(b) = velocity[b / v_div] (velocity == NULL: v_const); lx.n is the point count
-    const double* pts;
-    const double* velocity;
-    double v_const, dt;
-    int64_t v_div;
-};
 
 // FEET: the evaluation coordinates are the feet of the characteristics through the interpolation
 // points (computed here, not read), as in examples/characteristics_advection.cpp:243-250.
@@ -146,6 +130,7 @@ bool launch_build_eval_fused(BuildArgs const& args, Evaluator const& e, int orde
     fe.lx = lx;
     fe.out = out;
     fe.lo = lo;
+    if (launch_reg_fused(args, fe, order, false, s)) return true;
     int const kl = args.t.kl, ku = args.t.ku;
     if (kl == 1 && ku == 1) return launch_deg<1, 1>(args, fe, order, s);
     if (kl == 2 && ku == 2) return launch_deg<2, 2>(args, fe, order, s);
@@ -169,6 +154,7 @@ bool launch_advect_fused(BuildArgs const& args, Evaluator const& e, double const
     fe.v_const = v_const;
     fe.dt = dt;
     fe.v_div = v_div;
+    if (launch_reg_fused(args, fe, 0, true, s)) return true;
     int const kl = args.t.kl, ku = args.t.ku;
     if (kl == 1 && ku == 1) return launch_feet<1, 1>(args, fe, s);
     if (kl == 2 && ku == 2) return launch_feet<2, 2>(args, fe, s);

@@ -40,8 +40,11 @@ __global__ void __launch_bounds__(512, 1) reg_build_kernel(const __grid_constant
             reg_fill(args, io, (ti + gridDim.x) << (io.lp + 1), tile, raw);
         reg_sweeps<K, MINLEN>(t, sm, x, len, c, p, P);
         if (t.k > 0) reg_border(t, sm, x, a, len, c, p, P);
-        if (c < t.nchunk) reg_store(args, io, line, tile, a, len, p, x);
-        for (int r = c; r < t.k; r += nthr) reg_store_row(args, io, line, tile, t.m + r, p, sm.x2[r * P + p]);
+        if (c < t.nchunk) {
+            if (io.stage_out) reg_store_tile(args, io, tile, a, len, p, x);
+            else reg_store(args, line, a, len, x);
+        }
+        for (int r = c; r < t.k; r += nthr) reg_store_row(args, io, io.stage_out, line, tile, t.m + r, p, sm.x2[r * P + p]);
         if (io.stage_out) {
             __syncthreads();
             reg_drain(args, io, line0, tile);
@@ -64,11 +67,9 @@ template <int K>
 bool launch_reg(BuildArgs const& args, cudaStream_t s)
 {
     SolveTables const& t = args.t;
+    if (!reg_plain_rows(args)) return false;
     RegIo io {};
-    bool const all = args.raw || args.r.periodic;
-    io.v0 = all ? 0 : args.r.nbe_lo;
-    int const v1 = all ? t.n : args.r.nbe_lo + args.r.npoints;
-    if (args.r.lrot < io.v0 || args.r.lrot + t.m > v1) return false; // a row of Q that is no sample
+    io.v0 = (args.raw || args.r.periodic) ? 0 : args.r.nbe_lo;
     int dev = 0, optin = 0, sms = 0;
     DDCB_CUDA_CHECK(cudaGetDevice(&dev));
     DDCB_CUDA_CHECK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));

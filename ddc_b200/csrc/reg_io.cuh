@@ -23,6 +23,14 @@ struct RegIo
     int v0;         // row 0 of Q is system row lrot, sample lrot - v0 (the rows of Q are all samples)
 };
 
+// Whether every row of Q is a sample, one after the other (row 0 being sample lrot - v0).
+inline bool reg_plain_rows(BuildArgs const& args)
+{
+    bool const all = args.raw || args.r.periodic;
+    int const v0 = all ? 0 : args.r.nbe_lo, v1 = all ? args.t.n : args.r.nbe_lo + args.r.npoints;
+    return args.r.lrot >= v0 && args.r.lrot + args.t.m <= v1;
+}
+
 // The source of border row r (tile row m + r) of a line: a sample, a Hermite derivative, or none
 // (homogeneous conditions), and the power of dx that scales it.
 __device__ __forceinline__ const double* border_source(BuildArgs const& args, int r, int64_t line)
@@ -111,59 +119,62 @@ __device__ __forceinline__ void reg_border_rhs(BuildArgs const& args, RegSmem co
     for (int r = c; r < args.t.k; r += nthr) sm.b2[r * P + p] = mul2(*reinterpret_cast<const double2*>(raw + r * (2 * P) + 2 * p), border_scale(args, r));
 }
 
-// One row of the solution (tile order) of lines `line`, `line` + 1 to its coefficient row, and to the
-// row a period further that repeats it.
-__device__ __forceinline__ void reg_store_row(BuildArgs const& args, RegIo const& io, int64_t line, double* tile, int row, int p,
-                                              double2 v)
+// One border row of the solution (tile order) of a pair to its coefficient row and to the row a
+// period further that repeats it: in the tile, or in the coefficients of lines `line`, `line` + 1.
+__device__ __forceinline__ void reg_store_row(BuildArgs const& args, RegIo const& io, bool to_tile, int64_t line, double* tile, int row,
+                                              int p, double2 v)
 {
     int const n = args.t.n;
     int const rows = args.raw ? n : args.r.size;
     int o = row + args.r.srot;
     o -= (o >= n) ? n : 0;
     o += (o < 0) ? n : 0;
-    int const TL = 2 << io.lp;
-    double* const g0 = args.out + line_offset(args.lo, line);
-    double* const g1 = line + 1 < args.nlines ? args.out + line_offset(args.lo, line + 1) : nullptr;
     for (o = DDCB_INDEX(o, n); o < rows; o += n) {
-        if (io.stage_out) {
-            *reinterpret_cast<double2*>(tile + o * TL + 2 * p) = v;
+        if (to_tile) {
+            *reinterpret_cast<double2*>(tile + o * (2 << io.lp) + 2 * p) = v;
         } else if (line < args.nlines) {
-            __stcs(g0 + (int64_t)o * args.lo.stride, v.x);
-            if (g1) __stcs(g1 + (int64_t)o * args.lo.stride, v.y);
+            double* const g = args.out + (int64_t)o * args.lo.stride;
+            __stcs(g + line_offset(args.lo, line), v.x);
+            if (line + 1 < args.nlines) __stcs(g + line_offset(args.lo, line + 1), v.y);
         }
     }
 }
 
-// The rows [a, a + len) of the solution to the coefficients of lines `line`, `line` + 1: coefficient
-// rows a + srot .., from n on those from 0 on (the wrap of a periodic basis); rows below `dup` are
-// repeated n rows further. Only the chunks at the ends wrap or repeat, so the others are spared it.
-__device__ __forceinline__ void reg_store(BuildArgs const& args, RegIo const& io, int64_t line, double* tile, int a, int len, int p,
-                                          const double2* x)
+// The rows [a, a + len) of the solution to the tile, in coefficient order: rows a + srot .., from n on
+// those from 0 on (the wrap of a periodic basis); rows below `dup` are repeated n rows further.
+__device__ __forceinline__ void reg_store_tile(BuildArgs const& args, RegIo const& io, double* tile, int a, int len, int p,
+                                               const double2* x)
+{
+    int const n = args.t.n;
+    int const dup = (args.raw ? n : args.r.size) - n;
+    int o = a + args.r.srot;
+    o += (o < 0) ? n : 0;
+    int const TL = 2 << io.lp;
+    double* const t0 = tile + 2 * p;
+#pragma unroll
+    for (int s = 0; s < kRegRows; ++s)
+        if (s < len) {
+            int const q = o + s - (o + s >= n ? n : 0);
+            *reinterpret_cast<double2*>(t0 + q * TL) = x[s];
+            if (q < dup) *reinterpret_cast<double2*>(t0 + (q + n) * TL) = x[s];
+        }
+}
+
+// The same rows to the coefficients of lines `line`, `line` + 1. Only the chunks at the ends wrap or
+// repeat, so the others are spared it.
+__device__ __forceinline__ void reg_store(BuildArgs const& args, int64_t line, int a, int len, const double2* x)
 {
     constexpr int R = kRegRows;
     int const n = args.t.n;
     int const dup = (args.raw ? n : args.r.size) - n;
     int o = a + args.r.srot;
     o += (o < 0) ? n : 0;
-    bool const plain = o >= dup && o + len <= n;
-    if (io.stage_out) {
-        int const TL = 2 << io.lp;
-        double* const t0 = tile + 2 * p;
-#pragma unroll
-        for (int s = 0; s < R; ++s)
-            if (s < len) {
-                int const q = o + s - (o + s >= n ? n : 0);
-                *reinterpret_cast<double2*>(t0 + q * TL) = x[s];
-                if (q < dup) *reinterpret_cast<double2*>(t0 + (q + n) * TL) = x[s];
-            }
-        return;
-    }
     if (line >= args.nlines) return;
     int64_t const st = args.lo.stride;
     double* const base = args.out + line_offset(args.lo, line);
     bool const two = line + 1 < args.nlines;
     int64_t const next = two ? line_offset(args.lo, line + 1) - line_offset(args.lo, line) : 0;
-    if (plain) {
+    if (o >= dup && o + len <= n) {
         double* g = base + (int64_t)o * st;
         if (args.pair16_out) {
 #pragma unroll
@@ -201,7 +212,7 @@ __device__ __forceinline__ void reg_store(BuildArgs const& args, RegIo const& io
         }
 }
 
-// The tile's rows to the coefficients of unit-stride lines.
+// The tile's rows (coefficient order) to the coefficients.
 __device__ __forceinline__ void reg_drain(BuildArgs const& args, RegIo const& io, int64_t line0, const double* tile)
 {
     int const TL = 2 << io.lp;
@@ -209,8 +220,9 @@ __device__ __forceinline__ void reg_drain(BuildArgs const& args, RegIo const& io
     int const l = threadIdx.x & (TL - 1);
     int const step = blockDim.x / TL;
     if (line0 + l >= args.nlines) return;
+    int64_t const st = args.lo.stride;
     double* g = args.out + line_offset(args.lo, line0 + l);
-    for (int r = threadIdx.x / TL; r < rows; r += step) __stcs(g + r, tile[r * TL + l]);
+    for (int r = threadIdx.x / TL; r < rows; r += step) __stcs(g + r * st, tile[r * TL + l]);
 }
 
 } // namespace ddcb
