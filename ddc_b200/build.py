@@ -14,7 +14,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libddcb.so")
 LIB_CHECK = os.path.join(HERE, "libddcb_check.so")
-SOURCES = ["api.cu", "plan.cpp", "build_kernels.cu", "reg_build_kernels.cu", "reg_fused_kernels.cu", "eval_kernels.cu", "fused_kernels.cu", "tensor2d.cu",
+SOURCES = ["api.cu", "plan.cpp", "build_kernels.cu", "reg_build_kernels.cu", "reg_fused_kernels.cu", "reg_adjoint_kernels.cu", "eval_kernels.cu", "fused_kernels.cu", "tensor2d.cu",
            "adjoint_kernels.cu", "refine_kernels.cu",
            "uneven_batch.cu", "host_pipeline.cu", "quadrature.cu", "tensornd.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]

@@ -21,8 +21,7 @@
 #include <algorithm>
 #include <type_traits>
 
-#include "build_device.cuh"
-#include "eval_device.cuh"
+#include "adjoint_args.hpp"
 
 namespace ddcb {
 
@@ -54,24 +53,6 @@ struct RowsRotated
         int r = r0 + i;
         return r - ((r >= n) ? n : 0);
     }
-};
-
-struct AdjointArgs
-{
-    SolveTables t;          // factorisation of A^T
-    RhsMap r;
-    int64_t nlines;
-    int nct;
-    const double* gc;       // cotangents of the coefficients (size rows)
-    Lines lgc;
-    double* gv;             // cotangents of the samples (npoints rows)
-    Lines lgv;
-    double* gdlo;           // cotangents of the lower / upper Hermite derivatives (nbv rows), or NULL
-    Lines lglo;
-    double* gdhi;
-    Lines lghi;
-    int pair_in;            // g_coefs: adjacent line pairs 16-byte aligned and contiguous
-    int pair_out;           // g_vals: the same
 };
 
 // P^T: tile row j (column j of the solve) collects the cotangents of every coefficient row b with
@@ -190,25 +171,6 @@ __global__ void __launch_bounds__(1024) build_adjoint_kernel(const __grid_consta
     solve_in_tile<TL, KL, KU>(a.t, a.nct, smem);
     store_adjoint<TL>(a, smem);
 }
-
-struct EvalAdjointArgs
-{
-    EvalBasis eb;
-    int ex_lo, ex_hi;
-    int64_t nlines;
-    int size;               // coefficient rows
-    const double* coords;
-    Lines lx;
-    const double* coefs;    // needed for g_coords only
-    Lines lc;
-    int coef_pairs;         // coefs: adjacent line pairs 16-byte aligned and contiguous
-    const double* gy;       // cotangents of the evaluated values
-    Lines lgy;
-    double* gc;             // out: cotangents of the coefficients (standalone kernel)
-    Lines lgc;
-    double* gx;             // out: cotangents of the coordinates, or NULL
-    Lines lgx;
-};
 
 // The knot pairs (non-uniform bases) into shared memory, as async copies.
 template <bool UNI>
@@ -618,7 +580,8 @@ bool launch_build_eval_adjoint(Builder const& b, Evaluator const& e, int order, 
         a.nct = adj_nct(a.t, 8, kAdjThreads);
         EvalAdjointArgs ea = make_eval_adjoint_args(e, coords, lx, coefs, lc, gy, lgy, nullptr, Lines {}, gx, lgx);
         int const kl = a.t.kl, ku = a.t.ku;
-        if (kl == 1 && ku == 1) fused = launch_fused_deg<1, 1>(a, ea, order, s);
+        if (launch_reg_adjoint(a, ea, order, s)) fused = true;
+        else if (kl == 1 && ku == 1) fused = launch_fused_deg<1, 1>(a, ea, order, s);
         else if (kl == 2 && ku == 2) fused = launch_fused_deg<2, 2>(a, ea, order, s);
         else if (kl == 3 && ku == 3) fused = launch_fused_deg<3, 3>(a, ea, order, s);
         else if (kl == 4 && ku == 4) fused = launch_fused_deg<4, 4>(a, ea, order, s);

@@ -39,6 +39,18 @@ struct BasisDesc
     const double* knots; // non-uniform: ncells + 1 + 2*degree knots, knot k at knots[k]
 };
 
+// uniform_cell without branches, for kernels that keep several points in flight (the same numbers).
+DDCB_HD int uniform_cell_select(BasisDesc const& b, double x, double& offset)
+{
+    double o = (x - b.rmin) * b.inv_step;
+    int icell = static_cast<int>(o);
+    o = o - icell;
+    bool const low = x <= b.rmin, high = !low && (x >= b.rmax || icell >= b.ncells);
+    icell = low ? 0 : (high ? b.ncells - 1 : icell);
+    offset = low ? 0.0 : (high ? 1.0 : o);
+    return icell;
+}
+
 // bsplines_uniform.hpp:566-595. Returns the cell index and sets offset in [0,1].
 DDCB_HD int uniform_cell(BasisDesc const& b, double x, double& offset)
 {
@@ -255,11 +267,25 @@ DDCB_HD void uniform_values_raw(double offset, double* v)
 #pragma unroll
         for (int r = 1; r < j; ++r) {
             double const t = v[r];
-            v[r] = saved + above[r + 1] * t;
+            v[r] = fma(above[r + 1], t, saved); // explicit: every kernel rounds alike
             saved = below[j - 1 - r] * t;
         }
         v[j] = saved;
     }
+}
+
+// The raw values of degree P (times P!) and of degree P - 1 (times (P - 1)!) together.
+template <int P>
+DDCB_HD void uniform_values_raw2(double offset, double* v, double* vlow)
+{
+    uniform_values_raw<P - 1>(offset, vlow);
+    double saved = 0.0;
+#pragma unroll
+    for (int r = 0; r < P; ++r) {
+        v[r] = fma(r + 1 - offset, vlow[r], saved);
+        saved = (offset + (P - 1 - r)) * vlow[r];
+    }
+    v[P] = saved;
 }
 
 DDCB_HD constexpr double factorial_inverse(int p)

@@ -398,6 +398,46 @@ __device__ __forceinline__ double eval_deriv_no_bc(EvalBasis const& eb, double x
     return UNI && P > 1 ? y * factorial_inverse(P) : y;
 }
 
+// eval_point on uniform bases in two steps, so that a thread's points can first all be located (with
+// the rare branches of the boundary rules) and then evaluated side by side. uniform_place: the first
+// B-spline of x's cell and x's offset in it, -1 where the value is 0.
+template <int ORDER>
+__device__ __forceinline__ int uniform_place(EvalBasis const& eb, int ex_lo, int ex_hi, double x, double& off)
+{
+    bool zero = false;
+    if (ORDER == 0) {
+        if (eb.b.periodic) {
+            x = periodic_wrap(eb.b, x);
+        } else {
+            zero = (x < eb.b.rmin && ex_lo == 1) || (x > eb.b.rmax && ex_hi == 1);
+            // the constant rule evaluates at the domain end, which is what uniform_cell gives there
+        }
+    }
+    int const jmin = uniform_cell_select(eb.b, x, off);
+    return zero ? -1 : jmin;
+}
+
+template <int D, int ORDER, class Acc>
+__device__ __forceinline__ double uniform_at(EvalBasis const& eb, int jmin, double off, Acc const& C)
+{
+    constexpr int P = D - ORDER;
+    double v[P + 1], cc[D + 1];
+    uniform_values_raw<P>(off, v);
+    int const r0 = C.row0(DDCB_INDEX(jmin < 0 ? 0 : jmin, eb.b.ncells));
+#pragma unroll
+    for (int i = 0; i < D + 1; ++i) cc[i] = C.get(r0, i);
+#pragma unroll
+    for (int k = 1; k <= ORDER; ++k) {
+#pragma unroll
+        for (int i = D; i >= k; --i) cc[i] = (cc[i] - cc[i - 1]) * eb.b.inv_step;
+    }
+    double y = 0.0;
+#pragma unroll
+    for (int r = 0; r < P + 1; ++r) y = fma(cc[ORDER + r], v[r], y);
+    if (P > 1) y *= factorial_inverse(P);
+    return jmin < 0 ? 0.0 : y;
+}
+
 // Value (ORDER 0, with boundary handling) or ORDER-th derivative (no boundary handling).
 template <int D, int ORDER, bool UNI, class Acc>
 __device__ __forceinline__ double eval_point(EvalBasis const& eb, int ex_lo, int ex_hi, double x, Acc const& C)

@@ -119,15 +119,20 @@ __global__ void __launch_bounds__(kEvalThreads) eval_kernel(const __grid_constan
     CoefDirect const acc {C + l, TLE};
     // points in flight per thread: 16 for the derivative spline (its coordinates loaded together,
     // 0.78 -> 0.73 ms on 65536 quintic lines), 8 elsewhere (16 spills the other variants)
-    constexpr int U = DSPLINE ? 16 : 8;
+    constexpr int U = 8;
     int64_t const sx = a.lx.stride * nct, so = a.lo.stride * nct;
     const double* __restrict__ xp = a.coords + ox + c * a.lx.stride;
     double* __restrict__ op = a.out + oo + c * a.lo.stride;
     int const npt = m > c ? int((m - c + nct - 1) / nct) : 0; // points of this thread
-    for (int q0 = 0; q0 < npt; q0 += U) {
-        double xs[U];
+    auto load = [&](int q0, double* xs) {
 #pragma unroll
         for (int u = 0; u < U; ++u) xs[u] = (q0 + u < npt) ? __ldcs(xp + (q0 + u) * sx) : 0.0;
+    };
+    double xs[U];
+    load(0, xs);
+    for (int q0 = 0; q0 < npt; q0 += U) {
+        double next[U]; // on their way while this group is evaluated
+        load(q0 + U, next);
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             if (q0 + u >= npt) continue;
@@ -136,6 +141,8 @@ __global__ void __launch_bounds__(kEvalThreads) eval_kernel(const __grid_constan
             else y = eval_point<D, ORDER, UNI>(eb, a.ex_lo, a.ex_hi, xs[u], acc);
             __stcs(op + (q0 + u) * so, y);
         }
+#pragma unroll
+        for (int u = 0; u < U; ++u) xs[u] = next[u];
     }
 }
 

@@ -54,29 +54,42 @@ __global__ void __launch_bounds__(512, 1) reg_build_eval_kernel(const __grid_con
                 if (args.out != nullptr && args.pair16_out) reg_store_row(args, io, false, line0 + 2 * p, tile, t.m + r, p, sm.x2[r * P + p]);
             }
         }
+        // the first coordinates are on their way while the tile is completed, and each next group
+        // while the one before is evaluated
+        int64_t const line = min(line0 + l, args.nlines - 1);
+        int64_t const sx = fe.lx.stride * nct, so = fe.lo.stride * nct;
+        const double* __restrict__ xp = FEET ? fe.pts + q0 : fe.coords + line_offset(fe.lx, line) + q0 * fe.lx.stride;
+        double* __restrict__ op = fe.out + line_offset(fe.lo, line) + q0 * fe.lo.stride;
+        double const shift = FEET ? fe.dt * (fe.velocity ? __ldg(fe.velocity + line / fe.v_div) : fe.v_const) : 0.0;
+        CoefDirect const acc {tile + l, TL};
+        constexpr int U = 8; // points of a group
+        int const npt = m > q0 ? (m - q0 + nct - 1) / nct : 0;
+        auto load = [&](int i, double* xs) {
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (FEET) xs[u] = i + u < npt ? __ldg(xp + (i + u) * nct) : 0.0;
+                else xs[u] = i + u < npt ? __ldcs(xp + (i + u) * sx) : 0.0;
+            }
+        };
+        double xs[U];
+        load(0, xs);
         __syncthreads();
         if (args.out != nullptr && !args.pair16_out) reg_drain(args, io, line0, tile);
-        int64_t const line = line0 + l;
-        if (line < args.nlines) {
-            int64_t const sx = fe.lx.stride * nct, so = fe.lo.stride * nct;
-            const double* __restrict__ xp = FEET ? fe.pts + q0 : fe.coords + line_offset(fe.lx, line) + q0 * fe.lx.stride;
-            double* __restrict__ op = fe.out + line_offset(fe.lo, line) + q0 * fe.lo.stride;
-            double const shift = FEET ? fe.dt * (fe.velocity ? __ldg(fe.velocity + line / fe.v_div) : fe.v_const) : 0.0;
-            CoefDirect const acc {tile + l, TL};
-            constexpr int U = 8; // points in flight per thread
-            int const npt = m > q0 ? (m - q0 + nct - 1) / nct : 0;
+        if (line0 + l < args.nlines)
             for (int i = 0; i < npt; i += U) {
-                double xs[U];
+                double next[U];
+                load(i + U, next);
+                int j[U];
 #pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    if (FEET) xs[u] = i + u < npt ? __ldg(xp + (i + u) * nct) - shift : 0.0;
-                    else xs[u] = i + u < npt ? __ldcs(xp + (i + u) * sx) : 0.0;
-                }
+                for (int u = 0; u < U; ++u) j[u] = uniform_place<ORDER>(fe.eb, fe.ex_lo, fe.ex_hi, FEET ? xs[u] - shift : xs[u], xs[u]);
+#pragma unroll
+                for (int u = 0; u < U; ++u) xs[u] = uniform_at<D, ORDER>(fe.eb, j[u], xs[u], acc);
 #pragma unroll
                 for (int u = 0; u < U; ++u)
-                    if (i + u < npt) __stcs(op + (i + u) * so, eval_point<D, ORDER, true>(fe.eb, fe.ex_lo, fe.ex_hi, xs[u], acc));
+                    if (i + u < npt) __stcs(op + (i + u) * so, xs[u]);
+#pragma unroll
+                for (int u = 0; u < U; ++u) xs[u] = next[u];
             }
-        }
         __syncthreads();
     }
 }
