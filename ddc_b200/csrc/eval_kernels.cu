@@ -32,6 +32,7 @@ struct EvalArgs
     Lines lo;
     int pair16;         // coefs: adjacent line pairs 16-byte aligned and contiguous
     int lut_smem;       // non-uniform: bucket table copied to shared memory after the knot pairs
+    int row_ld, row_warps; // eval_rows_kernel: doubles between the lines in shared memory, lines per block
 };
 
 
@@ -146,9 +147,102 @@ __global__ void __launch_bounds__(kEvalThreads) eval_kernel(const __grid_constan
     }
 }
 
+// Lines whose own rows are contiguous (unit stride: coefficients, coordinates and values): a warp per
+// line. Lanes take neighbouring rows and points, so every access is a whole segment, and the line's
+// coefficients lie row after row in shared memory, where the neighbouring cells of neighbouring
+// points fall into different banks. The line-fastest tile of eval_kernel would read such arrays two
+// doubles per 32-byte sector (cubic values, 16384 x 1025 points: 138 us, here 88).
+template <int D, int ORDER, bool UNI>
+__global__ void __launch_bounds__(UNI ? 256 : 512, UNI ? 3 : 1) eval_rows_kernel(const __grid_constant__ EvalArgs a, int ld)
+{
+    extern __shared__ __align__(16) double smem[];
+    int const warps = blockDim.x / 32, w = threadIdx.x / 32, lane = threadIdx.x & 31;
+    double* const C = smem + w * ld;
+    double2* const K = reinterpret_cast<double2*>(smem + warps * ld);
+    double2* const L = K + a.eb.nk;
+    int64_t const line = (int64_t)blockIdx.x * warps + w;
+    if (line < a.nlines) {
+        const double* const g = a.coefs + line_offset(a.lc, line);
+        for (int r = lane; r < a.size; r += 32) cp_async8(C + r, g + r);
+    }
+    if (!UNI) {
+        for (int i = threadIdx.x; i < a.eb.nk - 1; i += blockDim.x) cp_async16(K + i, a.eb.kpairs + i);
+        if (a.lut_smem)
+            for (int i = threadIdx.x; i < a.eb.nbucket; i += blockDim.x) cp_async16(L + i, a.eb.lut + i);
+    }
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    __syncthreads();
+    if (line >= a.nlines) return;
+    constexpr bool DSPLINE = !UNI && ORDER == 1 && D >= 2;
+    if (DSPLINE) {
+        // the derivative spline's coefficients (eval_kernel), from the last rows to the first
+        const double* g = a.eb.inv_span + (size_t)(D - 1) * a.eb.nk;
+        for (int r0 = (a.size - 1) / 32 * 32; r0 >= 0; r0 -= 32) {
+            int const j = r0 + lane;
+            double const cj = j < a.size ? C[j] : 0.0, cp = j > 0 && j < a.size ? C[j - 1] : 0.0;
+            __syncwarp();
+            if (j < a.size) C[j] = j > 0 ? double(D) * (cj - cp) * __ldg(g + j) : 0.0;
+            __syncwarp();
+        }
+    }
+    EvalBasis eb = a.eb;
+    if (!UNI) {
+        eb.kpairs = K;
+        if (a.lut_smem) eb.lut = L;
+    }
+    const double* __restrict__ xp = a.coords + line_offset(a.lx, line) + lane;
+    double* __restrict__ op = a.out + line_offset(a.lo, line) + lane;
+    int const npt = int((a.lx.n - lane + 31) / 32);
+    CoefDirect const acc {C, 1};
+    constexpr int U = 4; // points of a group; the next group's coordinates are on their way meanwhile
+    auto load = [&](int q0, double* xs) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) xs[u] = q0 + u < npt ? __ldcs(xp + (q0 + u) * 32) : 0.0;
+    };
+    double xs[U];
+    load(0, xs);
+    for (int q0 = 0; q0 < npt; q0 += U) {
+        double next[U];
+        load(q0 + U, next);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (q0 + u >= npt) continue;
+            double y;
+            if constexpr (DSPLINE) y = nonuniform_deriv1_dcoef<D>(eb, xs[u], acc);
+            else y = eval_point<D, ORDER, UNI>(eb, a.ex_lo, a.ex_hi, xs[u], acc);
+            __stcs(op + (q0 + u) * 32, y);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) xs[u] = next[u];
+    }
+}
+
 template <int D, int TLE, bool UNI>
 void launch_order(EvalArgs const& a, int order, size_t sm, cudaStream_t s)
 {
+    if constexpr (TLE == 1) { // a warp per line
+        int const ld = a.row_ld, warps = a.row_warps;
+        size_t const bytes = sm;
+        dim3 rgrid((unsigned)((a.nlines + warps - 1) / warps)), rblock(32 * warps);
+#define DDCB_ROWS_CASE(O)                                                                                  \
+    case O:                                                                                                \
+        if constexpr (O <= D) {                                                                            \
+            auto k = eval_rows_kernel<D, O, UNI>;                                                          \
+            if (bytes > 48 * 1024) DDCB_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes))); \
+            k<<<rgrid, rblock, bytes, s>>>(a, ld);                                                         \
+        }                                                                                                  \
+        break;
+        switch (order) {
+            DDCB_ROWS_CASE(0)
+            DDCB_ROWS_CASE(1)
+            DDCB_ROWS_CASE(2)
+            DDCB_ROWS_CASE(3)
+            DDCB_ROWS_CASE(4)
+            DDCB_ROWS_CASE(5)
+        default: break;
+        }
+#undef DDCB_ROWS_CASE
+    } else {
     dim3 grid((unsigned)((a.nlines + TLE - 1) / TLE)), block(kEvalThreads);
 #define DDCB_EVAL_CASE(O)                                                                                  \
     case O:                                                                                                \
@@ -168,6 +262,7 @@ void launch_order(EvalArgs const& a, int order, size_t sm, cudaStream_t s)
     default: break;
     }
 #undef DDCB_EVAL_CASE
+    }
     DDCB_CUDA_CHECK(cudaGetLastError());
 }
 
@@ -226,6 +321,22 @@ void launch_eval(Evaluator const& e, int order, double* out, Lines const& lo, do
     int dev = 0, optin = 0;
     DDCB_CUDA_CHECK(cudaGetDevice(&dev));
     DDCB_CUDA_CHECK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    // unit-stride lines, enough of them to give every SM eight: a warp each
+    auto unit = [](Lines const& l) { return l.stride == 1 && l.inner == 1; };
+    int sms = 0;
+    DDCB_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    if (unit(lc) && unit(lx) && unit(lo) && a.nlines >= 8 * int64_t(sms) && lx.n < (int64_t(1) << 31)) {
+        a.row_ld = (a.size + 1) / 2 * 2;
+        for (int warps = uni ? 8 : 16; warps >= 4; warps /= 2)
+            for (int lut = uni ? 0 : 1; lut >= 0; --lut) {
+                size_t const b = bytes(warps, lut) + sizeof(double) * size_t(a.row_ld - a.size) * warps;
+                if (b > size_t(optin)) continue;
+                a.row_warps = warps;
+                a.lut_smem = lut;
+                launch_deg<1>(a, order, b, s);
+                return;
+            }
+    }
     for (int tle : {16, 8, 2})
         for (int lut = uni ? 0 : 1; lut >= 0; --lut)
             if (bytes(tle, lut) <= size_t(optin)) {
