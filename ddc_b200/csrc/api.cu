@@ -1038,17 +1038,19 @@ ddcb_status ddcb_build2d(ddcb_builder h1, ddcb_builder h2, double* coefs, const 
         cudaStream_t const s = reinterpret_cast<cudaStream_t>(stream);
         void* ws = workspace;
         bool owned = false;
+        int64_t group = 0; // as many fields at once as the build likes
         if (ws == nullptr) {
             DDCB_CUDA_CHECK(cudaMallocAsync(&ws, need, s));
             owned = true;
-        } else {
-            require(workspace_bytes >= need, "workspace too small (see ddcb_build2d_workspace_bytes)");
+        } else if (workspace_bytes < need) { // smaller groups of fields in a smaller workspace
+            group = ddcb::build2d_group_for(b1, b2, nbatch, workspace_bytes);
+            require(group > 0, "workspace too small (see ddcb_build2d_workspace_bytes)");
         }
         try {
             ddcb::launch_build2d(b1, b2, coefs, vals, h1lo ? dmin1 : nullptr, h1hi ? dmax1 : nullptr, h2lo ? dmin2 : nullptr,
                                  h2hi ? dmax2 : nullptr, (h1lo && h2lo) ? m11 : nullptr, (h1hi && h2lo) ? m21 : nullptr,
                                  (h1lo && h2hi) ? m12 : nullptr, (h1hi && h2hi) ? m22 : nullptr, nbatch,
-                                 static_cast<double*>(ws), s, 0, true);
+                                 static_cast<double*>(ws), s, group, true);
         } catch (...) {
             if (owned) cudaFreeAsync(ws, s);
             throw;

@@ -35,12 +35,22 @@ SideStream& side_stream_for_current_device()
 
 namespace {
 
-// Fields per group: the x1-pass result of a group stays near 40 MiB (L2-sized), and at most
-// max_group fields (0: no cap).
+int64_t field_bytes(Builder const& b1, Builder const& b2)
+{
+    return std::max<int64_t>(1, b1.basis.size() * int64_t(b2.points.size() + b2.nbv_lo + b2.nbv_hi) * 8);
+}
+
+// Fields whose x1-pass result stays near 40 MiB (L2-sized).
+int64_t l2_fields(Builder const& b1, Builder const& b2) { return std::max<int64_t>(1, (int64_t(40) << 20) / field_bytes(b1, b2)); }
+
+// Fields per group, at most max_group (0: no cap): 64 fields, whose rows are 512-byte segments in both
+// passes, while one group's x1-pass result stays below 256 MiB; else as many as stay L2-sized.
+// Narrower segments cost more than the second trip through HBM: 512^2 x 64 fields in groups of 16,
+// 32 and 64 build in 275, 249 and 229 us.
 int64_t group_fields(Builder const& b1, Builder const& b2, int64_t nbatch, int64_t max_group = 0)
 {
-    int64_t const per_field = b1.basis.size() * int64_t(b2.points.size() + b2.nbv_lo + b2.nbv_hi) * 8;
-    int64_t g = std::max<int64_t>(1, (int64_t(40) << 20) / std::max<int64_t>(per_field, 1));
+    int64_t g = l2_fields(b1, b2);
+    if (g < 64 && std::min<int64_t>(64, nbatch) * field_bytes(b1, b2) <= (int64_t(256) << 20)) g = 64;
     if (max_group > 0) g = std::min(g, max_group);
     return std::min(g, nbatch);
 }
@@ -58,6 +68,16 @@ size_t workspace_for_group(Builder const& b1, Builder const& b2, int64_t nbatch,
 size_t build2d_workspace_bytes(Builder const& b1, Builder const& b2, int64_t nbatch)
 {
     return workspace_for_group(b1, b2, nbatch, group_fields(b1, b2, nbatch));
+}
+
+// The widest group whose workspace fits in `bytes`; 0 below the workspace of the L2-sized group, which
+// is the least a caller has to bring.
+int64_t build2d_group_for(Builder const& b1, Builder const& b2, int64_t nbatch, size_t bytes)
+{
+    int64_t G = group_fields(b1, b2, nbatch);
+    int64_t const least = std::min(G, l2_fields(b1, b2));
+    while (G > least && workspace_for_group(b1, b2, nbatch, G) > bytes) --G;
+    return workspace_for_group(b1, b2, nbatch, G) <= bytes ? G : 0;
 }
 
 void launch_build2d(Builder const& b1, Builder const& b2, double* coefs, double const* vals, double const* dmin1,

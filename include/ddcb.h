@@ -314,14 +314,15 @@ ddcb_status ddcb_host_pipeline_run(ddcb_host_pipeline p, const double* vals, ddc
 /* ---- 2D tensor product: SplineBuilder2D / SplineEvaluator2D on two 1D plans, for the layout
  *      (x1, x2, batch) with the batch contiguous (the reference's layout_right of
  *      DiscreteDomain<X1, X2, batch...>). ----------------------------------------------------- */
-/* Workspace of ddcb_build2d: the x1-pass result of one group of fields. */
+/* Workspace of ddcb_build2d: the x1-pass result of one group of fields (up to 64 fields within
+ * 256 MiB). A smaller one, down to groups of about 40 MiB, is taken too and builds in more passes. */
 ddcb_status ddcb_build2d_workspace_bytes(ddcb_builder b1, ddcb_builder b2, int64_t nbatch, uint64_t* bytes);
 /* SplineBuilder2D::operator() (spline_builder_2d.hpp:455-651).
  *   vals (np1, np2, nbatch) -> coefs (size1, size2, nbatch);
  *   derivs_min1 / derivs_max1: (nbv1, np2, nbatch), read when b1's closure is HERMITE;
  *   derivs_min2 / derivs_max2: (np1, nbv2, nbatch), read when b2's closure is HERMITE;
  *   mixed_* (nbv1, nbv2, nbatch): cross derivatives at the four corners, read when both are HERMITE.
- * workspace: ddcb_build2d_workspace_bytes bytes of device memory, or NULL to have the call
+ * workspace: ddcb_build2d_workspace_bytes bytes of device memory (see there), or NULL to have the call
  * allocate it stream-ordered (cudaMallocAsync / cudaFreeAsync on `stream`). With Hermite
  * derivatives in dimension 2 the short derivative-slab passes run on a second stream of the
  * calling host thread, forked from and joined back to `stream` with events: the work stays ordered
