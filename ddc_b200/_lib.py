@@ -154,5 +154,13 @@ def check(status: int):
         raise DdcbError(status, msg)
 
 
+_entries = {}  # bound entry points, looked up once
+
+
 def call(name: str, *args):
-    check(getattr(load(), name)(*args))
+    f = _entries.get(name)
+    if f is None:
+        f = _entries[name] = getattr(load(), name)
+    status = f(*args)
+    if status:
+        check(status)

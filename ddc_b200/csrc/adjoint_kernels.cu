@@ -376,9 +376,7 @@ int adj_nct(SolveTables const& t, int TL, int min_threads)
 
 size_t optin_smem()
 {
-    int dev = 0, optin = 0;
-    DDCB_CUDA_CHECK(cudaGetDevice(&dev));
-    DDCB_CUDA_CHECK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    int const optin = device_limits().optin;
     return size_t(optin);
 }
 

@@ -17,6 +17,27 @@ struct ddcb_bsplines_t
 {
     ddcb::Basis basis;
 };
+namespace ddcb {
+
+DeviceLimits const& device_limits()
+{
+    constexpr int kDevices = 64;
+    static DeviceLimits limits[kDevices];
+    static std::once_flag once[kDevices];
+    int dev = 0;
+    DDCB_CUDA_CHECK(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= kDevices) throw Error(DDCB_ERR_UNSUPPORTED, "device ordinal above 63");
+    std::call_once(once[dev], [dev] {
+        DeviceLimits l;
+        DDCB_CUDA_CHECK(cudaDeviceGetAttribute(&l.optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+        DDCB_CUDA_CHECK(cudaDeviceGetAttribute(&l.sms, cudaDevAttrMultiProcessorCount, dev));
+        limits[dev] = l;
+    });
+    return limits[dev];
+}
+
+} // namespace ddcb
+
 struct ddcb_builder_t
 {
     ddcb::Builder* b;

@@ -298,9 +298,7 @@ __host__ __device__ inline size_t tile_doubles(SolveTables const& t, int TL, int
 template <class Bytes>
 inline int fit_tile_lines(int TL, Bytes bytes)
 {
-    int dev = 0, optin = 0;
-    DDCB_CUDA_CHECK(cudaGetDevice(&dev));
-    DDCB_CUDA_CHECK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    int const optin = device_limits().optin;
     for (int w = TL; w >= 2; w /= 2)
         if (bytes(w) <= size_t(optin)) return w;
     return TL;

@@ -29,9 +29,7 @@ void launch_tl(BuildArgs const& args, cudaStream_t s)
 {
     int const nct = args.nct;
     size_t const sm = smem_bytes(args.t, TL, KL, KU);
-    int dev = 0, optin = 0;
-    DDCB_CUDA_CHECK(cudaGetDevice(&dev));
-    DDCB_CUDA_CHECK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    int const optin = device_limits().optin;
     if (sm > size_t(optin))
         throw Error(DDCB_ERR_UNSUPPORTED, "line tile of " + std::to_string(sm) + " bytes exceeds shared memory (" + std::to_string(optin)
                                               + "); use fewer tile lines");
@@ -79,9 +77,7 @@ void dispatch(BuildArgs const& args, int TL, cudaStream_t s)
 // evaluates a whole tile alone (1000 lines: 28.9 -> 26.9 us).
 int fused_point_threads(int64_t nlines)
 {
-    int dev = 0, sms = 0;
-    DDCB_CUDA_CHECK(cudaGetDevice(&dev));
-    DDCB_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    int const sms = device_limits().sms;
     return (nlines + 7) / 8 < sms ? 128 : 64;
 }
 

@@ -28,6 +28,14 @@ struct Error : std::runtime_error
             throw ::ddcb::Error(DDCB_ERR_CUDA, std::string(#expr) + ": " + cudaGetErrorString(e_)); \
     } while (0)
 
+// What the launchers need to know of the current device, read from the runtime once per device
+// (api.cu): shared memory a block may opt in to, and the SM count.
+struct DeviceLimits
+{
+    int optin = 0, sms = 0;
+};
+DeviceLimits const& device_limits();
+
 // Strided batched array view: element (i, b) at base[i*stride + (b/inner)*outer_stride + b%inner].
 struct Lines
 {

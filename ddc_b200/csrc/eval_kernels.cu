@@ -318,13 +318,10 @@ void launch_eval(Evaluator const& e, int order, double* out, Lines const& lo, do
     auto bytes = [&](int tle, bool lut) {
         return sizeof(double) * ((size_t)a.size * tle + (uni ? 0 : 2 * ((size_t)e.eb.nk + (lut ? (size_t)e.eb.nbucket : 0))));
     };
-    int dev = 0, optin = 0;
-    DDCB_CUDA_CHECK(cudaGetDevice(&dev));
-    DDCB_CUDA_CHECK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    int const optin = device_limits().optin;
     // unit-stride lines, enough of them to give every SM eight: a warp each
     auto unit = [](Lines const& l) { return l.stride == 1 && l.inner == 1; };
-    int sms = 0;
-    DDCB_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    int const sms = device_limits().sms;
     if (unit(lc) && unit(lx) && unit(lo) && a.nlines >= 8 * int64_t(sms) && lx.n < (int64_t(1) << 31)) {
         a.row_ld = (a.size + 1) / 2 * 2;
         for (int warps = uni ? 8 : 16; warps >= 4; warps /= 2)

@@ -63,9 +63,7 @@ bool launch5(BuildArgs const& args, FusedEval const& fe, cudaStream_t s)
 {
     constexpr int TL = 8;
     size_t const sm = sizeof(double) * (tile_doubles(args.t, TL, KL, KU) + (UNI ? 0 : 2 * (size_t)fe.eb.nk + 2));
-    int dev = 0, optin = 0;
-    DDCB_CUDA_CHECK(cudaGetDevice(&dev));
-    DDCB_CUDA_CHECK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    int const optin = device_limits().optin;
     if (sm > size_t(optin)) return false;
     auto kern = build_eval_kernel<TL, KL, KU, D, ORDER, UNI, FEET>;
     if (sm > 48 * 1024) DDCB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));

@@ -691,25 +691,32 @@ struct HostSolve
         nscan_f = kl > 0 ? steps_needed(PhiF, kl) : 0;
         nscan_b = ku > 0 ? steps_needed(PhiB, ku) : 0;
         // The same bound chunk by chunk: a chunk's incoming carry needs the outgoing carries of the
-        // `t` chunks before it once every product of t transfers is below 2^-60.
-        auto chunks_needed = [&](std::vector<double> const& T, long K, bool fwd) -> long {
+        // `t` chunks before it once every product of t transfers is below 2^-60. The products of 1, 2
+        // and 4 are the scan's; those in between take one more multiplication.
+        auto chunks_needed = [&](std::vector<double> const& P, long K, bool fwd) -> long {
             if (K > 4) return 0; // wide bands: the scan
-            std::vector<double> prod(T), next(T.size());
-            for (long t = 1; t <= kDirectCarry; ++t) {
-                double mx = 0.0;
-                for (double v : prod) mx = std::max(mx, std::fabs(v));
-                if (mx <= 0x1p-60 || t >= nchunk - 1) return t;
+            std::vector<double> prod(K * K);
+            auto small = [&](long k, long k2) { // products of 2^k (and, behind them, of 2^k2) transfers
                 for (long c = 0; c < nchunk; ++c) {
-                    long const nb = fwd ? c - t : c + t;
-                    if (nb >= 0 && nb < nchunk) matmul(&prod[c * K * K], &T[nb * K * K], &next[c * K * K], K);
-                    else std::fill(&next[c * K * K], &next[c * K * K] + K * K, 0.0);
+                    double const* A = &P[(k * nchunk + c) * K * K];
+                    if (k2 >= 0) {
+                        long const nb = fwd ? c - (1L << k) : c + (1L << k);
+                        if (nb < 0 || nb >= nchunk) continue;
+                        matmul(A, &P[(k2 * nchunk + nb) * K * K], prod.data(), K);
+                        A = prod.data();
+                    }
+                    for (long q = 0; q < K * K; ++q)
+                        if (std::fabs(A[q]) > 0x1p-60) return false;
                 }
-                prod.swap(next);
-            }
+                return true;
+            };
+            static long const halves[kDirectCarry][2] = {{0, -1}, {1, -1}, {1, 0}, {2, -1}, {2, 0}, {2, 1}};
+            for (long t = 1; t <= kDirectCarry; ++t)
+                if (t >= nchunk - 1 || small(halves[t - 1][0], halves[t - 1][1])) return t;
             return 0;
         };
-        ndep_f = chunks_needed(F, kl, true);
-        ndep_b = chunks_needed(G, ku, false);
+        ndep_f = chunks_needed(PhiF, kl, true);
+        ndep_b = chunks_needed(PhiB, ku, false);
     }
 
     // Full host solve of A x = rhs (or A^T x = rhs): used for quadrature coefficients.

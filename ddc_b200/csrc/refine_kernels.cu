@@ -22,9 +22,7 @@ template <int TL, int KL, int KU>
 void launch_refine_tl(BuildArgs const& args, int rounds, cudaStream_t s)
 {
     size_t const sm = refine_smem(args.t, TL, KL, KU);
-    int dev = 0, optin = 0;
-    DDCB_CUDA_CHECK(cudaGetDevice(&dev));
-    DDCB_CUDA_CHECK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    int const optin = device_limits().optin;
     if (sm > size_t(optin))
         throw Error(DDCB_ERR_UNSUPPORTED, "refinement tile of " + std::to_string(sm) + " bytes exceeds shared memory; use fewer tile lines");
     auto kern = TL * args.nct <= 256 ? refine_kernel<TL, KL, KU, 256> : refine_kernel<TL, KL, KU, 1024>;

@@ -230,10 +230,7 @@ bool launch_kd(AdjointArgs const& a, EvalAdjointArgs const& ea, cudaStream_t s)
     SolveTables const& t = a.t;
     int const v0 = a.r.periodic ? 0 : a.r.nbe_lo, v1 = a.r.periodic ? t.n : a.r.nbe_lo + a.r.npoints;
     if (a.r.lrot < v0 || a.r.lrot + t.m > v1 || ea.lx.n > (int64_t(1) << 30)) return false;
-    int dev = 0, optin = 0, sms = 0;
-    DDCB_CUDA_CHECK(cudaGetDevice(&dev));
-    DDCB_CUDA_CHECK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    DDCB_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    int const optin = device_limits().optin, sms = device_limits().sms;
     int lp = 3;
     auto bytes = [&] { return sizeof(double) * (reg_smem_doubles<K>(t, 1 << lp) + size_t(t.n + ea.size) * size_t(2 << lp)); };
     auto fits = [&](int threads, int blocks) { return (t.nchunk << lp) <= threads && bytes() + 1024 <= (size_t(optin) + 1024) / blocks; };
@@ -246,9 +243,9 @@ bool launch_kd(AdjointArgs const& a, EvalAdjointArgs const& ea, cudaStream_t s)
     auto kern = full ? reg_adjoint_kernel<K, 15, D, ORDER> : reg_adjoint_kernel<K, 0, D, ORDER>;
     size_t const sm = bytes();
     DDCB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
-    int per_sm = 0;
-    DDCB_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, sm));
-    int64_t const grid = std::min<int64_t>(tiles(), int64_t(std::max(per_sm, 1)) * sms);
+    // resident blocks: 512 threads of 128 registers an SM, and the shared memory
+    int64_t const per_sm = std::max<int64_t>(1, std::min<int64_t>(512 / threads, (optin + 1024) / int64_t(sm + 1024)));
+    int64_t const grid = std::min<int64_t>(tiles(), per_sm * sms);
     kern<<<dim3((unsigned)grid), dim3((unsigned)threads), sm, s>>>(a, ea, lp);
     DDCB_CUDA_CHECK(cudaGetLastError());
     return true;

@@ -70,10 +70,7 @@ bool launch_reg(BuildArgs const& args, cudaStream_t s)
     if (!reg_plain_rows(args)) return false;
     RegIo io {};
     io.v0 = (args.raw || args.r.periodic) ? 0 : args.r.nbe_lo;
-    int dev = 0, optin = 0, sms = 0;
-    DDCB_CUDA_CHECK(cudaGetDevice(&dev));
-    DDCB_CUDA_CHECK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    DDCB_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    int const optin = device_limits().optin, sms = device_limits().sms;
     io.stage_out = args.lo.stride == 1 && args.lo.inner == 1 && args.lo.outer > 1;
     auto tiles = [&] { return (args.nlines + (int64_t(2) << io.lp) - 1) >> (io.lp + 1); };
     auto fits = [&](int threads, int blocks) {
@@ -100,9 +97,9 @@ bool launch_reg(BuildArgs const& args, cudaStream_t s)
     bool const full = t.nchunk > 1 && t.chunk_len >= 15;
     auto kern = full ? reg_build_kernel<K, 15> : reg_build_kernel<K, 0>;
     DDCB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
-    int per_sm = 0;
-    DDCB_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, bytes));
-    int64_t const grid = std::min<int64_t>(tiles(), int64_t(std::max(per_sm, 1)) * sms);
+    // resident blocks: 512 threads of 128 registers an SM, and the shared memory
+    int64_t const per_sm = std::max<int64_t>(1, std::min<int64_t>(512 / threads, (optin + 1024) / int64_t(bytes + 1024)));
+    int64_t const grid = std::min<int64_t>(tiles(), per_sm * sms);
     kern<<<dim3((unsigned)grid), dim3((unsigned)threads), bytes, s>>>(args, io);
     DDCB_CUDA_CHECK(cudaGetLastError());
     return true;

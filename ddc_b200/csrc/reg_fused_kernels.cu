@@ -101,10 +101,7 @@ bool launch_reg_fused_kd(BuildArgs const& args, FusedEval const& fe, cudaStream_
     if (!reg_plain_rows(args) || fe.lx.n > (int64_t(1) << 30)) return false;
     RegIo io {};
     io.v0 = args.r.periodic ? 0 : args.r.nbe_lo;
-    int dev = 0, optin = 0, sms = 0;
-    DDCB_CUDA_CHECK(cudaGetDevice(&dev));
-    DDCB_CUDA_CHECK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    DDCB_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    int const optin = device_limits().optin, sms = device_limits().sms;
     auto bytes = [&] { return sizeof(double) * (reg_smem_doubles<K>(t, 1 << io.lp) + size_t(args.r.size + t.k) * size_t(2 << io.lp)); };
     auto fits = [&](int threads, int blocks) { return (t.nchunk << io.lp) <= threads && bytes() + 1024 <= (size_t(optin) + 1024) / blocks; };
     auto tiles = [&] { return (args.nlines + (int64_t(2) << io.lp) - 1) >> (io.lp + 1); };
@@ -120,9 +117,9 @@ bool launch_reg_fused_kd(BuildArgs const& args, FusedEval const& fe, cudaStream_
     auto kern = full ? reg_build_eval_kernel<K, 15, D, ORDER, FEET> : reg_build_eval_kernel<K, 0, D, ORDER, FEET>;
     size_t const sm = bytes();
     DDCB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
-    int per_sm = 0;
-    DDCB_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, sm));
-    int64_t const grid = std::min<int64_t>(tiles(), int64_t(std::max(per_sm, 1)) * sms);
+    // resident blocks: 512 threads of 128 registers an SM, and the shared memory
+    int64_t const per_sm = std::max<int64_t>(1, std::min<int64_t>(512 / threads, (optin + 1024) / int64_t(sm + 1024)));
+    int64_t const grid = std::min<int64_t>(tiles(), per_sm * sms);
     kern<<<dim3((unsigned)grid), dim3((unsigned)threads), sm, s>>>(args, io, fe);
     DDCB_CUDA_CHECK(cudaGetLastError());
     return true;

@@ -273,9 +273,7 @@ namespace {
 
 int sm_count()
 {
-    int dev = 0, sms = 0;
-    DDCB_CUDA_CHECK(cudaGetDevice(&dev));
-    DDCB_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    int const sms = device_limits().sms;
     return sms;
 }
 

@@ -43,20 +43,36 @@ def n_boundary_equations(closure: int, degree: int) -> int:
     return degree // 2 if closure in (HERMITE, HOMOGENEOUS_HERMITE) else 0
 
 
-def _stream_handle(stream):
+def _torch_ops():
+    """torch, imported on the first device call (the plan-only classes work without it), and what a call needs of it."""
+    global _torch, _Tensor, _f64
     import torch
 
+    _torch, _Tensor, _f64 = torch, torch.Tensor, torch.float64
+    return torch
+
+
+_torch = _Tensor = _f64 = None
+
+
+def _stream_handle(stream):
     if stream is None:
-        stream = torch.cuda.current_stream()
-    return C.c_void_p(stream.cuda_stream)
+        stream = (_torch or _torch_ops()).cuda.current_stream()
+    return stream.cuda_stream
 
 
 def lines_of(t, dim: int) -> Lines:
     """ddcb_lines of tensor `t` with interest dimension `dim`; batch = all other dims (row-major)."""
-    shape = list(t.shape)
-    stride = list(t.stride())
+    shape = t.shape
+    stride = t.stride()
     nd = len(shape)
     dim = dim % nd if nd else 0
+    if nd == 2:  # one batch dimension: nothing to check but that a batch behind the rows is contiguous
+        n, b = shape[dim], shape[1 - dim]
+        if dim == 1:
+            return Lines(n, stride[1], 1, b, stride[0] if b > 1 else 0)
+        if b <= 1 or stride[1] == 1:
+            return Lines(n, stride[0], b, 1, 0)
     n = shape[dim] if nd else 1
     inner_dims = list(range(dim + 1, nd))
     outer_dims = list(range(0, dim))
@@ -79,15 +95,15 @@ def lines_of(t, dim: int) -> Lines:
 
 
 def _ptr(t):
-    return C.c_void_p(0 if t is None else t.data_ptr())
+    return 0 if t is None else t.data_ptr()
 
 
 def _dev_f64(t, name):
-    import torch
-
     if t is None:
         return None
-    if not (isinstance(t, torch.Tensor) and t.is_cuda and t.dtype == torch.float64):
+    if _torch is None:
+        _torch_ops()
+    if not (isinstance(t, _Tensor) and t.is_cuda and t.dtype == _f64):
         raise TypeError(f"{name} must be a CUDA float64 tensor")
     return t
 
