@@ -17,22 +17,45 @@
 namespace ddcb {
 
 
-// W = float(b - A X) for the tile's lines; ends with a barrier.
+// W = float(b - A X) for the tile's lines; ends with a barrier. A thread takes every step-th row of a
+// pair of lines (of the one line of a TL = 1 tile), kResidualRows at a time: their right-hand sides
+// come from global memory and are all under way before the first sum, and an entry of A serves both
+// lines. (512 cells x 8192 lines, two rounds: the one-row loop waited for the L2 once per row.)
+constexpr int kResidualRows = 4;
+
 template <int TL>
 __device__ __forceinline__ void residual_tile(BuildArgs const& args, const double* X, float* W)
 {
+    using V = Lanes<double, TL>;
+    using F = Lanes<float, TL>;
+    constexpr int P = TL % 2 == 0 ? TL / 2 : 1;
     SolveTables const& t = args.t;
     int const n = t.n;
-    int const l = threadIdx.x % TL;
-    int const c = threadIdx.x / TL;
-    int const nct = blockDim.x / TL;
-    int64_t const line = tile_line0<TL>(args) + l;
-    bool const live = line < args.nlines;
-    for (int r = c; r < n; r += nct) {
-        double s = live ? rhs_row(args, r, line) : 0.0;
-        int const q1 = __ldg(t.a_row + r + 1);
-        for (int q = __ldg(t.a_row + r); q < q1; ++q) s = fma(-__ldg(t.a_val + q), X[__ldg(t.a_col + q) * TL + l], s);
-        W[r * TL + l] = float(s);
+    int const p = threadIdx.x % P;
+    int const c = threadIdx.x / P;
+    int const step = blockDim.x / P;
+    int64_t const line = tile_line0<TL>(args) + (TL % 2 == 0 ? 2 : 1) * p;
+    bool const live0 = line < args.nlines, live1 = TL % 2 == 0 && line + 1 < args.nlines;
+    const V* const X2 = reinterpret_cast<const V*>(X) + p;
+    F* const W2 = reinterpret_cast<F*>(W) + p;
+    for (int r0 = c; r0 < n; r0 += kResidualRows * step) {
+        V s[kResidualRows];
+#pragma unroll
+        for (int u = 0; u < kResidualRows; ++u) {
+            int const r = r0 + u * step;
+            double const b0 = live0 && r < n ? rhs_row(args, r, line) : 0.0;
+            if constexpr (TL % 2 == 0) s[u] = make_double2(b0, live1 && r < n ? rhs_row(args, r, line + 1) : 0.0);
+            else s[u] = b0;
+        }
+#pragma unroll
+        for (int u = 0; u < kResidualRows; ++u) {
+            int const r = r0 + u * step;
+            if (r >= n) break;
+            int const q1 = __ldg(t.a_row + r + 1);
+            for (int q = __ldg(t.a_row + r); q < q1; ++q) s[u] = fma2(-__ldg(t.a_val + q), X2[__ldg(t.a_col + q) * P], s[u]);
+            if constexpr (TL % 2 == 0) W2[r * P] = make_float2(float(s[u].x), float(s[u].y));
+            else W2[r * P] = float(s[u]);
+        }
     }
     __syncthreads();
 }
