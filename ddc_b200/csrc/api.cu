@@ -135,22 +135,26 @@ Evaluator* create_evaluator(Basis const& basis, int ex_lo, int ex_hi)
             for (int i = 0; i + len < nk; ++i) ispan[size_t(len - 1) * nk + i] = inv(i, i + len);
         // bucket table over nb uniform buckets, at least one per cell and, up to 4 per cell and
         // 4096 in all, no wider than the narrowest cell, so that a bucket holds at most one knot:
-        // {split, c0} with c0 the cell holding the bucket start and split the first knot inside
-        // the bucket (+inf if none)
+        // the first knot inside the bucket (+inf if none), its low bits (16; 24 or 31 on meshes of
+        // more cells) replaced by the cell holding the bucket start
         int const last = d + D.ncells - 1;
         double hmin = D.rmax - D.rmin;
         for (int cc = d; cc <= last; ++cc) hmin = std::min(hmin, t[cc + 1] - t[cc]);
         double const want = std::ceil((D.rmax - D.rmin) / hmin);
         int const nb = std::max(std::max(1, D.ncells),
                                 int(std::min(want, double(std::min(4 * std::max(1, D.ncells), 4096)))));
-        std::vector<double> lut(size_t(2) * nb);
+        uint64_t const mask = last < 0x10000 ? 0xFFFFu : (last < 0x1000000 ? 0xFFFFFFu : 0x7FFFFFFFu);
+        std::vector<double> lut(static_cast<size_t>(nb));
         double const scale = double(nb) / (D.rmax - D.rmin);
         int c = d;
         for (int bk = 0; bk < nb; ++bk) {
             double const x0 = D.rmin + double(bk) / scale, x1 = D.rmin + double(bk + 1) / scale;
             while (c < last && x0 >= t[c + 1]) ++c;
-            lut[2 * size_t(bk)] = (c < last && t[c + 1] < x1) ? t[c + 1] : HUGE_VAL;
-            lut[2 * size_t(bk) + 1] = double(c);
+            double const split = (c < last && t[c + 1] < x1) ? t[c + 1] : HUGE_VAL;
+            uint64_t bits = 0;
+            std::memcpy(&bits, &split, 8);
+            bits = (bits & ~mask) | uint64_t(c);
+            std::memcpy(&lut[size_t(bk)], &bits, 8);
         }
         e->integrals.resize(e->basis.size());
         basis_integrals(e->basis, e->integrals.data());
@@ -172,7 +176,8 @@ Evaluator* create_evaluator(Basis const& basis, int ex_lo, int ex_hi)
         e->d_integrals = reinterpret_cast<double*>(base + o_int);
         e->eb.b = e->basis.device_desc();
         e->eb.kpairs = reinterpret_cast<double2 const*>(base);
-        e->eb.lut = reinterpret_cast<double2 const*>(base + o_lut);
+        e->eb.lut = reinterpret_cast<double const*>(base + o_lut);
+        e->eb.lut_mask = int(mask);
         e->eb.inv_span = reinterpret_cast<double const*>(base + o_isp);
         e->eb.nbucket = nb;
         e->eb.bucket_scale = scale;

@@ -19,9 +19,10 @@ struct EvalBasis
     const double2* kpairs;    // nk-1 pairs (t_i, t_i+1): device copy, or shared-memory copy in a kernel
     const double* inv_span;   // degree x nk: inv_span[(len-1)*nk + i] = 1/(t[i+len] - t[i]) (0 if empty);
                               // global memory, or a shared-memory copy in a kernel (plain loads)
-    const double2* lut;       // nbucket entries {split, c0}: c0 the cell (knot index) holding the
-                              // bucket start, split the first knot inside the bucket (+inf if none);
-                              // device copy, or shared-memory copy in a kernel
+    const double* lut;        // nbucket entries: the first knot inside the bucket (none: +inf), its low
+                              // mantissa bits replaced by the cell (knot index) holding the bucket
+                              // start; device copy, or shared-memory copy in a kernel
+    int lut_mask;             // those bits
     int nbucket;
     double bucket_scale;      // nbucket / (rmax - rmin)
     int nk;                   // number of knots
@@ -77,7 +78,9 @@ struct CoefGlobal
 // the end rules of bsplines_non_uniform.hpp:666-695: the bucket's start cell, plus one past the
 // bucket's inner knot. Exact when the bucket holds at most one knot (the table is built with
 // buckets no wider than the narrowest cell, up to a size cap) and x is not within rounding of a
-// bucket edge; nonuniform_walk finishes it otherwise.
+// bucket edge or of the knot; nonuniform_walk finishes it otherwise. One 8-byte entry holds both
+// numbers: random 16-byte shared loads cost 10 wavefronts a warp, 8-byte ones 6, and the cell needs
+// no conversion.
 __device__ __forceinline__ int nonuniform_guess(EvalBasis const& eb, double x)
 {
     int const d = eb.b.degree;
@@ -85,8 +88,8 @@ __device__ __forceinline__ int nonuniform_guess(EvalBasis const& eb, double x)
     if (x >= eb.b.rmax) return d + eb.b.ncells - 1;
     int bk = static_cast<int>((x - eb.b.rmin) * eb.bucket_scale);
     bk = bk < 0 ? 0 : (bk >= eb.nbucket ? eb.nbucket - 1 : bk);
-    double2 const e = eb.lut[bk];
-    return static_cast<int>(e.y) + (x >= e.x ? 1 : 0);
+    double const e = eb.lut[bk];
+    return (__double2loint(e) & eb.lut_mask) + (x >= e ? 1 : 0); // (+inf with cell bits is a NaN: no knot, false)
 }
 
 // Whether c is the cell of x, given tc = t_c and tc1 = t_c+1.

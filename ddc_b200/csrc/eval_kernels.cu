@@ -82,11 +82,11 @@ __global__ void __launch_bounds__(kEvalThreads) eval_kernel(const __grid_constan
         int64_t const oc = line_offset(a.lc, line);
         for (int r = c; r < a.size; r += nct) cp_async8(C + r * TLE + l, a.coefs + r * a.lc.stride + oc);
     }
-    double2* L = K + a.eb.nk; // bucket table (non-uniform, lut_smem)
+    double* L = reinterpret_cast<double*>(K + a.eb.nk); // bucket table (non-uniform, lut_smem)
     if (!UNI) {
         for (int i = tid; i < a.eb.nk - 1; i += blockDim.x) cp_async16(K + i, a.eb.kpairs + i);
         if (a.lut_smem)
-            for (int i = tid; i < a.eb.nbucket; i += blockDim.x) cp_async16(L + i, a.eb.lut + i);
+            for (int i = 2 * tid; i < a.eb.nbucket; i += 2 * blockDim.x) cp_async16(L + i, a.eb.lut + i);
     }
     asm volatile("cp.async.wait_all;\n" ::: "memory");
     __syncthreads();
@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(UNI ? 256 : 512, UNI ? 3 : 1) eval_rows_kernel
     int const warps = blockDim.x / 32, w = threadIdx.x / 32, lane = threadIdx.x & 31;
     double* const C = smem + w * ld;
     double2* const K = reinterpret_cast<double2*>(smem + warps * ld);
-    double2* const L = K + a.eb.nk;
+    double* const L = reinterpret_cast<double*>(K + a.eb.nk);
     int64_t const line = (int64_t)blockIdx.x * warps + w;
     if (line < a.nlines) {
         const double* const g = a.coefs + line_offset(a.lc, line);
@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(UNI ? 256 : 512, UNI ? 3 : 1) eval_rows_kernel
     if (!UNI) {
         for (int i = threadIdx.x; i < a.eb.nk - 1; i += blockDim.x) cp_async16(K + i, a.eb.kpairs + i);
         if (a.lut_smem)
-            for (int i = threadIdx.x; i < a.eb.nbucket; i += blockDim.x) cp_async16(L + i, a.eb.lut + i);
+            for (int i = 2 * threadIdx.x; i < a.eb.nbucket; i += 2 * blockDim.x) cp_async16(L + i, a.eb.lut + i);
     }
     asm volatile("cp.async.wait_all;\n" ::: "memory");
     __syncthreads();
@@ -316,7 +316,7 @@ void launch_eval(Evaluator const& e, int order, double* out, Lines const& lo, do
     // memory when it fits too
     bool const uni = e.eb.b.uniform != 0;
     auto bytes = [&](int tle, bool lut) {
-        return sizeof(double) * ((size_t)a.size * tle + (uni ? 0 : 2 * ((size_t)e.eb.nk + (lut ? (size_t)e.eb.nbucket : 0))));
+        return sizeof(double) * ((size_t)a.size * tle + (uni ? 0 : 2 * ((size_t)e.eb.nk + (lut ? ((size_t)e.eb.nbucket + 1) / 2 : 0))));
     };
     int const optin = device_limits().optin;
     // unit-stride lines, enough of them to give every SM eight: a warp each
