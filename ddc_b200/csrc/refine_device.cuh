@@ -18,16 +18,20 @@ namespace ddcb {
 
 
 // W = float(b - A X) for the tile's lines; ends with a barrier. A thread takes every step-th row of a
-// pair of lines (of the one line of a TL = 1 tile), kResidualRows at a time: their right-hand sides
+// pair of lines, four at a time: their right-hand sides
 // come from global memory and are all under way before the first sum, and an entry of A serves both
-// lines. (512 cells x 8192 lines, two rounds: the one-row loop waited for the L2 once per row.)
-constexpr int kResidualRows = 4;
+// lines. (512 cells x 8192 lines, two rounds: the one-row loop waited for the L2 once per row, 182
+// against 172 us.) One-line tiles keep one row at a time: their many small blocks hide the wait, and
+// the registers of four rows would cost them residency.
+template <int TL>
+constexpr int residual_rows() { return TL % 2 == 0 ? 4 : 1; }
 
 template <int TL>
 __device__ __forceinline__ void residual_tile(BuildArgs const& args, const double* X, float* W)
 {
     using V = Lanes<double, TL>;
     using F = Lanes<float, TL>;
+    constexpr int kResidualRows = residual_rows<TL>();
     constexpr int P = TL % 2 == 0 ? TL / 2 : 1;
     SolveTables const& t = args.t;
     int const n = t.n;
