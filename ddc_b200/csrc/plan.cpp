@@ -711,6 +711,7 @@ struct HostSolve
                 return true;
             };
             static long const halves[kDirectCarry][2] = {{0, -1}, {1, -1}, {1, 0}, {2, -1}, {2, 0}, {2, 1}};
+            if (nchunk - 1 > kDirectCarry && !small(2, 1)) return 0; // too far for all of them
             for (long t = 1; t <= kDirectCarry; ++t)
                 if (t >= nchunk - 1 || small(halves[t - 1][0], halves[t - 1][1])) return t;
             return 0;
@@ -1285,6 +1286,7 @@ void upload_builder(Builder* b)
     b->device = dev;
     upload_basis(b->basis, dev);
     std::vector<char> blob;
+    blob.reserve(size_t(b->n) * 1024 + 65536); // both systems' tables: grown once, not copied along
     std::vector<size_t> offs_f, offs_a;
     b->tables = upload_tables(priv->fwd, blob, offs_f);
     b->tables_t = upload_tables(priv->adj, blob, offs_a);
