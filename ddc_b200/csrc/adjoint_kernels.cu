@@ -380,19 +380,13 @@ size_t optin_smem()
     return size_t(optin);
 }
 
-template <class Kern>
-void set_smem(Kern k, size_t sm)
-{
-    if (sm > 48 * 1024) DDCB_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
-}
-
 template <int TL, int KL, int KU>
 void launch_build_adjoint_tl(AdjointArgs const& a, cudaStream_t s)
 {
     size_t const sm = sizeof(double) * tile_doubles(a.t, TL, KL, KU);
     if (sm > optin_smem()) throw Error(DDCB_ERR_UNSUPPORTED, "adjoint line tile exceeds shared memory; use fewer tile lines");
     auto kern = build_adjoint_kernel<TL, KL, KU>;
-    set_smem(kern, sm);
+    allow_shared(kern, sm);
     kern<<<dim3((unsigned)((a.nlines + TL - 1) / TL)), dim3(TL * a.nct), sm, s>>>(a);
     DDCB_CUDA_CHECK(cudaGetLastError());
 }
@@ -482,11 +476,11 @@ void launch_eval_adjoint_d(EvalAdjointArgs const& a, int order, cudaStream_t s)
     dim3 grid((unsigned)((a.nlines + TLE - 1) / TLE)), block(kAdjThreads);
     if (order == 0) {
         auto k = eval_adjoint_kernel<D, TLE, 0, UNI>;
-        set_smem(k, sm);
+        allow_shared(k, sm);
         k<<<grid, block, sm, s>>>(a);
     } else {
         auto k = eval_adjoint_kernel<D, TLE, 1, UNI>;
-        set_smem(k, sm);
+        allow_shared(k, sm);
         k<<<grid, block, sm, s>>>(a);
     }
     DDCB_CUDA_CHECK(cudaGetLastError());
@@ -513,7 +507,7 @@ bool launch_fused5(AdjointArgs const& a, EvalAdjointArgs const& ea, cudaStream_t
     size_t const sm = sizeof(double) * fused_tile_doubles(a.t, ea.size, TL, KL, KU) + (UNI ? 0 : sizeof(double2) * (size_t)ea.eb.nk);
     if (sm > optin_smem()) return false;
     auto kern = build_eval_adjoint_kernel<TL, KL, KU, D, ORDER, UNI>;
-    set_smem(kern, sm);
+    allow_shared(kern, sm);
     kern<<<dim3((unsigned)((a.nlines + TL - 1) / TL)), dim3(TL * a.nct), sm, s>>>(a, ea);
     DDCB_CUDA_CHECK(cudaGetLastError());
     return true;

@@ -36,7 +36,7 @@ void launch_tl(BuildArgs const& args, cudaStream_t s)
     auto kern = TL == 16 ? build_kernel<TL, KL, KU, 512>
                          : (TL * nct <= 256 ? build_kernel<TL, KL, KU, 256> : build_kernel<TL, KL, KU, 1024>);
     if (TL == 16 && TL * nct > 512) throw Error(DDCB_ERR_UNSUPPORTED, "16-line tiles take at most 32 chunk threads per line");
-    if (sm > 48 * 1024) DDCB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
+    allow_shared(kern, sm);
     int64_t const grid = (args.nlines + TL - 1) / TL;
     kern<<<dim3((unsigned)grid), dim3(TL * nct), sm, s>>>(args);
     DDCB_CUDA_CHECK(cudaGetLastError());

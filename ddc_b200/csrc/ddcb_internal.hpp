@@ -36,6 +36,19 @@ struct DeviceLimits
 };
 DeviceLimits const& device_limits();
 
+#if defined(__CUDACC__)
+// Lets `kern` take `bytes` of dynamic shared memory. The limit belongs to the kernel on the device,
+// not to the launch that sets it: every launch that needs one sets the same, the most the kernel can
+// have beside its `fixed` static bytes, so that a small launch of another host thread, between this
+// call and the launch it is for, cannot lower it.
+template <class Kern>
+void allow_shared(Kern kern, size_t bytes, size_t fixed = 0)
+{
+    if (bytes > 48 * 1024)
+        DDCB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(size_t(device_limits().optin) - fixed)));
+}
+#endif
+
 // Strided batched array view: element (i, b) at base[i*stride + (b/inner)*outer_stride + b%inner].
 struct Lines
 {

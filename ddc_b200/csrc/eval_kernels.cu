@@ -228,7 +228,7 @@ void launch_order(EvalArgs const& a, int order, size_t sm, cudaStream_t s)
     case O:                                                                                                \
         if constexpr (O <= D) {                                                                            \
             auto k = eval_rows_kernel<D, O, UNI>;                                                          \
-            if (bytes > 48 * 1024) DDCB_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes))); \
+            allow_shared(k, bytes); \
             k<<<rgrid, rblock, bytes, s>>>(a, ld);                                                         \
         }                                                                                                  \
         break;
@@ -248,7 +248,7 @@ void launch_order(EvalArgs const& a, int order, size_t sm, cudaStream_t s)
     case O:                                                                                                \
         if constexpr (O <= D) {                                                                            \
             auto k = eval_kernel<D, TLE, O, UNI>;                                                          \
-            if (sm > 48 * 1024) DDCB_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm))); \
+            allow_shared(k, sm); \
             k<<<grid, block, sm, s>>>(a);                                                                  \
         }                                                                                                  \
         break;

@@ -66,7 +66,7 @@ bool launch5(BuildArgs const& args, FusedEval const& fe, cudaStream_t s)
     int const optin = device_limits().optin;
     if (sm > size_t(optin)) return false;
     auto kern = build_eval_kernel<TL, KL, KU, D, ORDER, UNI, FEET>;
-    if (sm > 48 * 1024) DDCB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
+    allow_shared(kern, sm);
     int64_t const grid = (args.nlines + TL - 1) / TL;
     kern<<<dim3((unsigned)grid), dim3(TL * args.nct), sm, s>>>(args, fe);
     DDCB_CUDA_CHECK(cudaGetLastError());

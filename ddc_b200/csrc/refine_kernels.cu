@@ -26,7 +26,7 @@ void launch_refine_tl(BuildArgs const& args, int rounds, cudaStream_t s)
     if (sm > size_t(optin))
         throw Error(DDCB_ERR_UNSUPPORTED, "refinement tile of " + std::to_string(sm) + " bytes exceeds shared memory; use fewer tile lines");
     auto kern = TL * args.nct <= 256 ? refine_kernel<TL, KL, KU, 256> : refine_kernel<TL, KL, KU, 1024>;
-    if (sm > 48 * 1024) DDCB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
+    allow_shared(kern, sm);
     int64_t const grid = (args.nlines + TL - 1) / TL;
     kern<<<dim3((unsigned)grid), dim3(TL * args.nct), sm, s>>>(args, rounds);
     DDCB_CUDA_CHECK(cudaGetLastError());

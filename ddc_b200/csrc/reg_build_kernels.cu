@@ -96,7 +96,7 @@ bool launch_reg(BuildArgs const& args, cudaStream_t s)
     // no chunk shorter than 15 rows: tests on the last two steps only
     bool const full = t.nchunk > 1 && t.chunk_len >= 15;
     auto kern = full ? reg_build_kernel<K, 15> : reg_build_kernel<K, 0>;
-    DDCB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
+    allow_shared(kern, bytes);
     // resident blocks: 512 threads of 128 registers an SM, and the shared memory
     int64_t const per_sm = std::max<int64_t>(1, std::min<int64_t>(512 / threads, (optin + 1024) / int64_t(bytes + 1024)));
     int64_t const grid = std::min<int64_t>(tiles(), per_sm * sms);

@@ -116,7 +116,7 @@ bool launch_reg_fused_kd(BuildArgs const& args, FusedEval const& fe, cudaStream_
     bool const full = t.nchunk > 1 && t.chunk_len >= 15;
     auto kern = full ? reg_build_eval_kernel<K, 15, D, ORDER, FEET> : reg_build_eval_kernel<K, 0, D, ORDER, FEET>;
     size_t const sm = bytes();
-    DDCB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
+    allow_shared(kern, sm);
     // resident blocks: 512 threads of 128 registers an SM, and the shared memory
     int64_t const per_sm = std::max<int64_t>(1, std::min<int64_t>(512 / threads, (optin + 1024) / int64_t(sm + 1024)));
     int64_t const grid = std::min<int64_t>(tiles(), per_sm * sms);
