@@ -40,10 +40,12 @@ struct BasisDesc
 };
 
 // uniform_cell without branches, for kernels that keep several points in flight (the same numbers).
+// A NaN is in no comparison and converts to a negative integer on the device: cell 0, with a NaN offset.
 DDCB_HD int uniform_cell_select(BasisDesc const& b, double x, double& offset)
 {
     double o = (x - b.rmin) * b.inv_step;
     int icell = static_cast<int>(o);
+    icell = icell < 0 ? 0 : icell;
     o = o - icell;
     bool const low = x <= b.rmin, high = !low && (x >= b.rmax || icell >= b.ncells);
     icell = low ? 0 : (high ? b.ncells - 1 : icell);
@@ -64,6 +66,7 @@ DDCB_HD int uniform_cell(BasisDesc const& b, double x, double& offset)
     } else {
         offset = (x - b.rmin) * b.inv_step;
         icell = static_cast<int>(offset);
+        if (icell < 0) icell = 0; // a NaN: it stays one, in a cell of the basis
         offset = offset - icell;
         // The reference maps icell == ncells with a zero offset to the last cell. The scaled
         // offset can also round to just above ncells for x a few ulps below rmax; that point is

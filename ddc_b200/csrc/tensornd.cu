@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(kThreadsNd) evalnd_kernel(const __grid_constan
                 if (a.eb[d].b.periodic) x[d] = periodic_wrap(a.eb[d].b, x[d]);
             for (int d = 0; d < N && !done; ++d) {
                 BasisDesc const& bd = a.eb[d].b;
-                if (bd.periodic || (x[d] >= bd.rmin && x[d] <= bd.rmax)) continue;
+                if (bd.periodic || !(x[d] < bd.rmin || x[d] > bd.rmax)) continue; // a NaN stays one
                 bool const low = x[d] < bd.rmin;
                 if ((low ? a.ex_lo[d] : a.ex_hi[d]) == DDCB_EXTRAP_NULL) {
                     y = 0.0;
@@ -277,7 +277,7 @@ __device__ __forceinline__ bool place3d(EvalNdArgs const& a, double* x)
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         BasisDesc const& bd = a.eb[d].b;
-        if (bd.periodic || (x[d] >= bd.rmin && x[d] <= bd.rmax)) continue;
+        if (bd.periodic || !(x[d] < bd.rmin || x[d] > bd.rmax)) continue; // a NaN stays one
         bool const low = x[d] < bd.rmin;
         if ((low ? a.ex_lo[d] : a.ex_hi[d]) == DDCB_EXTRAP_NULL) return false;
         x[d] = low ? bd.rmin : bd.rmax;
