@@ -48,7 +48,8 @@ def _torch_ops():
     global _torch, _Tensor, _f64
     import torch
 
-    _torch, _Tensor, _f64 = torch, torch.Tensor, torch.float64
+    _Tensor, _f64 = torch.Tensor, torch.float64
+    _torch = torch  # last: other threads take it for the sign that all are there
     return torch
 
 
