@@ -270,16 +270,20 @@ __device__ __forceinline__ void carry_scan(const R* __restrict__ Pm, V* C2, int 
 }
 
 // The true carry leaving chunk b (0 outside the line): read where the scan has left it (nd = 0), or
-// chained here from its neighbours' outgoing carries.
+// chained here from its neighbours' outgoing carries. Plans chain bands of up to kDirectBand only, and
+// the wider ones must not carry the code: its 64 matrix entries an unrolled step made kernels of bands
+// of eight spill some 1500 bytes a thread (64 registers), for a path they never took.
 template <class R, class V, int K, int KC, bool FWD>
 __device__ __forceinline__ void carry_of(const R* __restrict__ Pm, const V* C2, int P, int nd, int NC, int b, V* out)
 {
 #pragma unroll
     for (int q = 0; q < K; ++q) out[q] = zero_of<V>();
     if (b < 0 || b >= NC) return;
-    if (nd > 0) {
-        carry_direct<V, K, KC, FWD>([&](int c, int e) { return __ldg(Pm + e * NC + c); }, C2, P, nd, NC, b, out);
-        return;
+    if constexpr (K <= kDirectBand) {
+        if (nd > 0) {
+            carry_direct<V, K, KC, FWD>([&](int c, int e) { return __ldg(Pm + e * NC + c); }, C2, P, nd, NC, b, out);
+            return;
+        }
     }
 #pragma unroll
     for (int q = 0; q < K; ++q) out[q] = C2[(b * KC + q) * P];

@@ -694,7 +694,7 @@ struct HostSolve
         // `t` chunks before it once every product of t transfers is below 2^-60. The products of 1, 2
         // and 4 are the scan's; those in between take one more multiplication.
         auto chunks_needed = [&](std::vector<double> const& P, long K, bool fwd) -> long {
-            if (K > 4) return 0; // wide bands: the scan
+            if (K > kDirectBand) return 0; // the scan
             std::vector<double> prod(K * K);
             auto small = [&](long k, long k2) { // products of 2^k (and, behind them, of 2^k2) transfers
                 for (long c = 0; c < nchunk; ++c) {
@@ -1230,7 +1230,6 @@ Builder* create_builder_host(Basis const& basis, double const* pts, long npts, i
         }
         priv->fwd.analyse(rows, D.periodic != 0, top + bottom);
         priv->fwd.make_tables(b->nchunk_req);
-        priv->adj.analyse(transpose_rows(rows), D.periodic != 0, top + bottom);
         priv->adj.make_tables(b->nchunk_req);
         b->k = int(priv->fwd.k);
         b->m = int(priv->fwd.m);
