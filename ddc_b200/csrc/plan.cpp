@@ -1230,6 +1230,7 @@ Builder* create_builder_host(Basis const& basis, double const* pts, long npts, i
         }
         priv->fwd.analyse(rows, D.periodic != 0, top + bottom);
         priv->fwd.make_tables(b->nchunk_req);
+        priv->adj.analyse(transpose_rows(rows), D.periodic != 0, top + bottom);
         priv->adj.make_tables(b->nchunk_req);
         b->k = int(priv->fwd.k);
         b->m = int(priv->fwd.m);
