@@ -40,17 +40,17 @@ struct BasisDesc
 };
 
 // uniform_cell without branches, for kernels that keep several points in flight (the same numbers).
-// A NaN is in no comparison and converts to a negative integer on the device: cell 0, with a NaN offset.
+// A NaN fails every comparison and converts to a negative integer on the device; as unsigned that is
+// beyond the last cell, which it gets, with its offset left NaN.
 DDCB_HD int uniform_cell_select(BasisDesc const& b, double x, double& offset)
 {
     double o = (x - b.rmin) * b.inv_step;
     int icell = static_cast<int>(o);
-    icell = icell < 0 ? 0 : icell;
     o = o - icell;
     bool const low = x <= b.rmin, high = !low && (x >= b.rmax || icell >= b.ncells);
-    icell = low ? 0 : (high ? b.ncells - 1 : icell);
+    unsigned const last = static_cast<unsigned>(b.ncells - 1), cell = static_cast<unsigned>(icell);
     offset = low ? 0.0 : (high ? 1.0 : o);
-    return icell;
+    return low ? 0 : static_cast<int>(cell < last ? cell : last);
 }
 
 // bsplines_uniform.hpp:566-595. Returns the cell index and sets offset in [0,1].
@@ -66,15 +66,14 @@ DDCB_HD int uniform_cell(BasisDesc const& b, double x, double& offset)
     } else {
         offset = (x - b.rmin) * b.inv_step;
         icell = static_cast<int>(offset);
-        if (icell < 0) icell = 0; // a NaN: it stays one, in a cell of the basis
         offset = offset - icell;
         // The reference maps icell == ncells with a zero offset to the last cell. The scaled
         // offset can also round to just above ncells for x a few ulps below rmax; that point is
         // the end of the last cell too (the reference would index past its coefficients there).
-        if (icell >= b.ncells) {
-            icell = b.ncells - 1;
-            offset = 1.0;
-        }
+        // A NaN (a negative icell on the device) gets that cell too, and stays one.
+        if (icell >= b.ncells) offset = 1.0;
+        unsigned const cell = static_cast<unsigned>(icell), last = static_cast<unsigned>(b.ncells - 1);
+        icell = static_cast<int>(cell < last ? cell : last);
     }
     return icell;
 }
