@@ -149,6 +149,7 @@ struct SolveTables
 // before it (no scan, no barrier); slower decays run the log-depth scan.
 constexpr int kDirectCarry = 6;
 constexpr int kDirectBand = 4;     // and only for bands of at most this many sub- or super-diagonals
+constexpr int kTileChunks = 64;    // chunks a line of the shared-memory tile is cut into by default
 constexpr int kRegRows = 17;       // rows of one chunk that a thread holds in registers
 constexpr int kRegMaxChunks = 128; // chunks of the longest line the register solve takes: tiles of
                                    // eight lines (four pairs) within 512 threads

@@ -18,20 +18,15 @@ namespace ddcb {
 
 
 // W = float(b - A X) for the tile's lines; ends with a barrier. A thread takes every step-th row of a
-// pair of lines, four at a time: their right-hand sides
-// come from global memory and are all under way before the first sum, and an entry of A serves both
-// lines. (512 cells x 8192 lines, two rounds: the one-row loop waited for the L2 once per row, 182
-// against 172 us.) One-line tiles keep one row at a time: their many small blocks hide the wait, and
-// the registers of four rows would cost them residency.
-template <int TL>
-constexpr int residual_rows() { return TL % 2 == 0 ? 4 : 1; }
-
+// pair of lines, so that an entry of A serves both. One row at a time: what hides the wait for the
+// right-hand side is the other warps, and four rows in flight took the registers of half of them (cubic
+// Hermite on an irregular mesh, 512 cells x 8192 lines: 182 us; one row, with the blocks that fit
+// then, 113).
 template <int TL>
 __device__ __forceinline__ void residual_tile(BuildArgs const& args, const double* X, float* W)
 {
     using V = Lanes<double, TL>;
     using F = Lanes<float, TL>;
-    constexpr int kResidualRows = residual_rows<TL>();
     constexpr int P = TL % 2 == 0 ? TL / 2 : 1;
     SolveTables const& t = args.t;
     int const n = t.n;
@@ -42,24 +37,15 @@ __device__ __forceinline__ void residual_tile(BuildArgs const& args, const doubl
     bool const live0 = line < args.nlines, live1 = TL % 2 == 0 && line + 1 < args.nlines;
     const V* const X2 = reinterpret_cast<const V*>(X) + p;
     F* const W2 = reinterpret_cast<F*>(W) + p;
-    for (int r0 = c; r0 < n; r0 += kResidualRows * step) {
-        V s[kResidualRows];
-#pragma unroll
-        for (int u = 0; u < kResidualRows; ++u) {
-            int const r = r0 + u * step;
-            double const b0 = live0 && r < n ? rhs_row(args, r, line) : 0.0;
-            if constexpr (TL % 2 == 0) s[u] = make_double2(b0, live1 && r < n ? rhs_row(args, r, line + 1) : 0.0);
-            else s[u] = b0;
-        }
-#pragma unroll
-        for (int u = 0; u < kResidualRows; ++u) {
-            int const r = r0 + u * step;
-            if (r >= n) break;
-            int const q1 = __ldg(t.a_row + r + 1);
-            for (int q = __ldg(t.a_row + r); q < q1; ++q) s[u] = fma2(-__ldg(t.a_val + q), X2[__ldg(t.a_col + q) * P], s[u]);
-            if constexpr (TL % 2 == 0) W2[r * P] = make_float2(float(s[u].x), float(s[u].y));
-            else W2[r * P] = float(s[u]);
-        }
+    for (int r = c; r < n; r += step) {
+        V s;
+        double const b0 = live0 ? rhs_row(args, r, line) : 0.0;
+        if constexpr (TL % 2 == 0) s = make_double2(b0, live1 ? rhs_row(args, r, line + 1) : 0.0);
+        else s = b0;
+        int const q1 = __ldg(t.a_row + r + 1);
+        for (int q = __ldg(t.a_row + r); q < q1; ++q) s = fma2(-__ldg(t.a_val + q), X2[__ldg(t.a_col + q) * P], s);
+        if constexpr (TL % 2 == 0) W2[r * P] = make_float2(float(s.x), float(s.y));
+        else W2[r * P] = float(s);
     }
     __syncthreads();
 }

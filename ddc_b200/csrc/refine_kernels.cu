@@ -9,9 +9,10 @@ namespace ddcb {
 
 namespace {
 
-// MAXT: the largest block the instantiation takes (blocks of up to 256 threads get 128 registers).
-template <int TL, int KL, int KU, int MAXT>
-__global__ void __launch_bounds__(MAXT, MAXT <= 256 ? 2 : 1) refine_kernel(const __grid_constant__ BuildArgs args, int rounds)
+// MAXT: the largest block the instantiation takes; MINB: the blocks of that size an SM holds (of 256
+// threads: two of up to 128 registers, or four of 64).
+template <int TL, int KL, int KU, int MAXT, int MINB>
+__global__ void __launch_bounds__(MAXT, MINB) refine_kernel(const __grid_constant__ BuildArgs args, int rounds)
 {
     extern __shared__ __align__(16) double smem[];
     refine_tile<TL, KL, KU>(args, smem, rounds);
@@ -25,9 +26,16 @@ void launch_refine_tl(BuildArgs const& args, int rounds, cudaStream_t s)
     int const optin = device_limits().optin;
     if (sm > size_t(optin))
         throw Error(DDCB_ERR_UNSUPPORTED, "refinement tile of " + std::to_string(sm) + " bytes exceeds shared memory; use fewer tile lines");
-    auto kern = TL * args.nct <= 256 ? refine_kernel<TL, KL, KU, 256> : refine_kernel<TL, KL, KU, 1024>;
-    allow_shared(kern, sm);
+    auto kern = TL * args.nct <= 256 ? refine_kernel<TL, KL, KU, 256, 2> : refine_kernel<TL, KL, KU, 1024, 1>;
     int64_t const grid = (args.nlines + TL - 1) / TL;
+    // Four blocks an SM instead of two where the tiles leave room for a third and the batch has the
+    // blocks: their waits hide each other's (cubic Hermite on an irregular mesh, 512 cells x 8192
+    // lines: 113 us with 64 registers, 164 with 128). With fewer blocks the registers are free
+    // (1000 cells x 8192 lines: 298 against 272). Bands of four spill too much in 64.
+    if constexpr (TL == 8 && KU <= 3)
+        if (TL * args.nct <= 256 && (size_t(optin) + 1024) / (sm + 1024) >= 3 && grid > 2 * int64_t(device_limits().sms))
+            kern = refine_kernel<TL, KL, KU, 256, 4>;
+    allow_shared(kern, sm);
     kern<<<dim3((unsigned)grid), dim3(TL * args.nct), sm, s>>>(args, rounds);
     DDCB_CUDA_CHECK(cudaGetLastError());
 }
