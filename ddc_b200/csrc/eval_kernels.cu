@@ -118,9 +118,12 @@ __global__ void __launch_bounds__(kEvalThreads) eval_kernel(const __grid_constan
     int64_t const oo = line_offset(a.lo, line);
     int64_t const m = a.lx.n;
     CoefDirect const acc {C + l, TLE};
-    // points in flight per thread: 16 for the derivative spline (its coordinates loaded together,
-    // 0.78 -> 0.73 ms on 65536 quintic lines), 8 elsewhere (16 spills the other variants)
+    // A thread's points go in groups of eight, the next group's coordinates on their way meanwhile
+    // (cubic values on an irregular mesh, 256 cells x 8192 lines: 28.8 against 32.9 us). Not where
+    // those registers cost more than the wait: on irregular meshes linear splines (18.6 against 24.7),
+    // quintic values (39.1 against 41.1) and most higher derivatives (quartic, second: 37.7 against 43.2).
     constexpr int U = 8;
+    constexpr bool AHEAD = UNI || (D >= 2 && (ORDER == 0 ? D < 5 : ORDER == 1 || (ORDER == 2 && D == 5)));
     int64_t const sx = a.lx.stride * nct, so = a.lo.stride * nct;
     const double* __restrict__ xp = a.coords + ox + c * a.lx.stride;
     double* __restrict__ op = a.out + oo + c * a.lo.stride;
@@ -130,10 +133,10 @@ __global__ void __launch_bounds__(kEvalThreads) eval_kernel(const __grid_constan
         for (int u = 0; u < U; ++u) xs[u] = (q0 + u < npt) ? __ldcs(xp + (q0 + u) * sx) : 0.0;
     };
     double xs[U];
-    load(0, xs);
+    if (AHEAD) load(0, xs);
     for (int q0 = 0; q0 < npt; q0 += U) {
-        double next[U]; // on their way while this group is evaluated
-        load(q0 + U, next);
+        double next[U];
+        load(AHEAD ? q0 + U : q0, AHEAD ? next : xs);
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             if (q0 + u >= npt) continue;
@@ -142,10 +145,19 @@ __global__ void __launch_bounds__(kEvalThreads) eval_kernel(const __grid_constan
             else y = eval_point<D, ORDER, UNI>(eb, a.ex_lo, a.ex_hi, xs[u], acc);
             __stcs(op + (q0 + u) * so, y);
         }
+        if (AHEAD) {
 #pragma unroll
-        for (int u = 0; u < U; ++u) xs[u] = next[u];
+            for (int u = 0; u < U; ++u) xs[u] = next[u];
+        }
     }
 }
+
+// The fewest warps an SM with which a warp per line still beats the line tiles (us, 4096 lines; 2048
+// from 2750 cells on). Uniform cubic values: 12 warps at 2048 cells 58 against 84 in tiles, 11 at 2300
+// 78 against 79, 10 at 2500 85 against 82; first derivatives, with less to compute: 9 at 3000 cells 45
+// against 51, 8 at 3500 cells 60 against 72, 7 at 4096 cells 72 against 65. Irregular meshes keep the
+// knots beside the lines: 16 warps at 1500 cells 86 against 124, 14 at 1750 cells 101 against 88.
+inline int row_warps_needed(bool uni, int order) { return !uni ? 16 : (order == 0 ? 12 : 8); }
 
 // Lines whose own rows are contiguous (unit stride: coefficients, coordinates and values): a warp per
 // line. Lanes take neighbouring rows and points, so every access is a whole segment, and the line's
@@ -319,20 +331,31 @@ void launch_eval(Evaluator const& e, int order, double* out, Lines const& lo, do
         return sizeof(double) * ((size_t)a.size * tle + (uni ? 0 : 2 * ((size_t)e.eb.nk + (lut ? ((size_t)e.eb.nbucket + 1) / 2 : 0))));
     };
     int const optin = device_limits().optin;
-    // unit-stride lines, enough of them to give every SM eight: a warp each
+    // unit-stride lines, enough of them to give every SM eight: a warp each. Every warp keeps a whole
+    // line in shared memory, so the blocks are made smaller where that lets at least a fifth more warps
+    // run (2048 cells: two blocks of 6 instead of one of 8; registers allow 24 warps, or 16 with irregular
+    // meshes)
     auto unit = [](Lines const& l) { return l.stride == 1 && l.inner == 1; };
     int const sms = device_limits().sms;
     if (unit(lc) && unit(lx) && unit(lo) && a.nlines >= 8 * int64_t(sms) && lx.n < (int64_t(1) << 31)) {
         a.row_ld = (a.size + 1) / 2 * 2;
-        for (int warps = uni ? 8 : 16; warps >= 4; warps /= 2)
+        int most = 0;
+        size_t row_bytes = 0;
+        for (int warps = uni ? 8 : 16; warps >= 4; --warps)
             for (int lut = uni ? 0 : 1; lut >= 0; --lut) {
                 size_t const b = bytes(warps, lut) + sizeof(double) * size_t(a.row_ld - a.size) * warps;
                 if (b > size_t(optin)) continue;
+                int const run = std::min(int((size_t(optin) + 1024) / (b + 1024)) * warps, (uni ? 24 : 16) / warps * warps);
+                if (5 * run < 6 * most || run <= most) continue;
+                most = run;
+                row_bytes = b;
                 a.row_warps = warps;
                 a.lut_smem = lut;
-                launch_deg<1>(a, order, b, s);
-                return;
             }
+        if (most >= row_warps_needed(uni, order)) {
+            launch_deg<1>(a, order, row_bytes, s);
+            return;
+        }
     }
     for (int tle : {16, 8, 2})
         for (int lut = uni ? 0 : 1; lut >= 0; --lut)
