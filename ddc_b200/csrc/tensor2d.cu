@@ -14,6 +14,7 @@
 
 #include "build_device.cuh"
 #include "eval_device.cuh"
+#include "tensor_items.cuh"
 
 namespace ddcb {
 
@@ -206,46 +207,34 @@ __device__ __forceinline__ V eval2d_point(Eval2dArgs const& a, double x1, double
     return scale == 1.0 ? y : mul2(y, scale);
 }
 
-constexpr int kThreads2d = 256;
-constexpr int kItems2d = 2048; // (point, field) items per block, over at most 32 columns
-
-// A block evaluates ppb consecutive points for hs of the H columns of fields: single fields, or
-// (PAIR) pairs of neighbouring fields, which share basis and position and load their coefficients as
-// 16-byte vectors where their points coincide (feet computed once for all fields), else take turns.
-// Items are numbered point by point, so few fields fill a warp with several points.
+// A block evaluates items of single fields, or (PAIR) of pairs of neighbouring fields, which share basis
+// and position and load their coefficients as 16-byte vectors where their points coincide (feet
+// computed once for all fields).
 template <int D1, int D2, int O1, int O2, bool U1, bool U2, bool PAIR>
-__global__ void __launch_bounds__(kThreads2d) eval2d_kernel(const __grid_constant__ Eval2dArgs a, int ppb, int H, int hs)
+__global__ void __launch_bounds__(kItemThreads) eval2d_kernel(const __grid_constant__ Eval2dArgs a, int ppb, int H, int hs)
 {
-    int const h0 = blockIdx.y * hs;
-    hs = min(hs, H - h0);
-    int64_t const p0 = (int64_t)blockIdx.x * ppb;
-    int const np = int(min((int64_t)ppb, a.m - p0));
-    int q = threadIdx.x / hs, h = threadIdx.x - q * hs;
-    int const dq = kThreads2d / hs, dh = kThreads2d - dq * hs;
-    while (q < np) {
-        int64_t const at = (p0 + q) * a.B + (PAIR ? 2 : 1) * (h0 + h);
-        const double* const C = a.coefs + (PAIR ? 2 : 1) * (h0 + h);
-        const double2* const xy = reinterpret_cast<const double2*>(a.coords) + at;
-        double2 const u = __ldcs(xy);
-        if constexpr (PAIR) {
-            double2 const w = __ldcs(xy + 1);
-            double2 y;
-            if (u.x == w.x && u.y == w.y) {
-                y = eval2d_point<D1, D2, O1, O2, U1, U2, double2>(a, u.x, u.y, C);
-            } else {
-                y.x = eval2d_point<D1, D2, O1, O2, U1, U2, double>(a, u.x, u.y, C);
-                y.y = eval2d_point<D1, D2, O1, O2, U1, U2, double>(a, w.x, w.y, C + 1);
-            }
-            __stcs(reinterpret_cast<double2*>(a.out + at), y);
-        } else {
-            __stcs(a.out + at, eval2d_point<D1, D2, O1, O2, U1, U2, double>(a, u.x, u.y, C));
-        }
-        q += dq;
-        h += dh;
-        if (h >= hs) {
-            h -= hs;
-            ++q;
-        }
+    const double2* const xy = reinterpret_cast<const double2*>(a.coords);
+    if constexpr (PAIR) {
+        for_items<true>(a.m, ppb, H, hs, [&](bool live, int64_t p, int h) {
+            int64_t const at = p * a.B + 2 * h;
+            double2 const u = __ldcs(xy + at), w = __ldcs(xy + at + 1);
+            pair_items(
+                live, at, h, u.x == w.x && u.y == w.y,
+                [&](int64_t to, int c) {
+                    __stcs(reinterpret_cast<double2*>(a.out + to),
+                           eval2d_point<D1, D2, O1, O2, U1, U2, double2>(a, u.x, u.y, a.coefs + 2 * c));
+                },
+                [&](int64_t to, int field) {
+                    double2 const v = __ldcs(xy + to);
+                    __stcs(a.out + to, eval2d_point<D1, D2, O1, O2, U1, U2, double>(a, v.x, v.y, a.coefs + field));
+                });
+        });
+    } else {
+        for_items<false>(a.m, ppb, H, hs, [&](int64_t p, int h) {
+            int64_t const at = p * a.B + h;
+            double2 const u = __ldcs(xy + at);
+            __stcs(a.out + at, eval2d_point<D1, D2, O1, O2, U1, U2, double>(a, u.x, u.y, a.coefs + h));
+        });
     }
 }
 
@@ -253,10 +242,9 @@ template <int D1, int D2, int O1, int O2, bool U1, bool U2>
 void launch_eval2d_p(Eval2dArgs const& a, cudaStream_t s)
 {
     bool const pair = a.B % 2 == 0 && reinterpret_cast<uintptr_t>(a.coefs) % 16 == 0 && reinterpret_cast<uintptr_t>(a.out) % 16 == 0;
-    int const H = int(pair ? a.B / 2 : a.B), hs = std::min(H, 32), ppb = kItems2d / hs;
-    dim3 const grid((unsigned)((a.m + ppb - 1) / ppb), (unsigned)((H + hs - 1) / hs));
-    if (pair) eval2d_kernel<D1, D2, O1, O2, U1, U2, true><<<grid, kThreads2d, 0, s>>>(a, ppb, H, hs);
-    else eval2d_kernel<D1, D2, O1, O2, U1, U2, false><<<grid, kThreads2d, 0, s>>>(a, ppb, H, hs);
+    ItemGrid const g = item_grid(a.m, a.B, pair);
+    if (pair) eval2d_kernel<D1, D2, O1, O2, U1, U2, true><<<g.grid, kItemThreads, 0, s>>>(a, g.ppb, g.H, g.hs);
+    else eval2d_kernel<D1, D2, O1, O2, U1, U2, false><<<g.grid, kItemThreads, 0, s>>>(a, g.ppb, g.H, g.hs);
     DDCB_CUDA_CHECK(cudaGetLastError());
 }
 

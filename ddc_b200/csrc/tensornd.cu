@@ -25,6 +25,7 @@
 
 #include "build_device.cuh"
 #include "eval_device.cuh"
+#include "tensor_items.cuh"
 
 namespace ddcb {
 
@@ -129,9 +130,6 @@ void launch_build3d(Builder const& b1, Builder const& b2, Builder const& b3, dou
 // ---------------------------------------------------------------------------------------------
 namespace {
 
-constexpr int kThreadsNd = 256;
-constexpr int kItemsNd = 2048; // (point, batch entry) items per block, over at most 32 columns
-
 struct EvalNdArgs
 {
     int ndims;
@@ -200,32 +198,10 @@ __device__ double tensor_sum(EvalNdArgs const& a, const double* C, const int* jm
     return y;
 }
 
-// The (point, column) items of a block: ppb consecutive points, hs of the H columns, numbered point by
-// point, so that few batch entries fill a warp with several points. f(point, column).
-template <class F>
-__device__ __forceinline__ void for_items(int64_t m, int ppb, int H, int hs, F f)
-{
-    int const h0 = blockIdx.y * hs;
-    hs = min(hs, H - h0);
-    int64_t const p0 = (int64_t)blockIdx.x * ppb;
-    int const np = int(min((int64_t)ppb, m - p0));
-    int q = threadIdx.x / hs, h = threadIdx.x - q * hs;
-    int const dq = kThreadsNd / hs, dh = kThreadsNd - dq * hs;
-    while (q < np) {
-        f(p0 + q, h0 + h);
-        q += dq;
-        h += dh;
-        if (h >= hs) {
-            h -= hs;
-            ++q;
-        }
-    }
-}
-
-__global__ void __launch_bounds__(kThreadsNd) evalnd_kernel(const __grid_constant__ EvalNdArgs a, int ppb, int H, int hs)
+__global__ void __launch_bounds__(kItemThreads) evalnd_kernel(const __grid_constant__ EvalNdArgs a, int ppb, int H, int hs)
 {
     int const N = a.ndims;
-    for_items(a.m, ppb, H, hs, [&](int64_t p, int b) {
+    for_items<false>(a.m, ppb, H, hs, [&](int64_t p, int b) {
         const double* C = a.coefs + b;
         const double* xp = a.coords + (p * a.B + b) * N;
         double x[kMaxDims];
@@ -338,39 +314,41 @@ __device__ __forceinline__ V eval3d_point(EvalNdArgs const& a, double x0, double
 }
 
 // Columns are batch entries, or (PAIR) pairs of neighbouring ones, which share the basis and load
-// their coefficients as 16-byte vectors where their points coincide, and take turns where not.
+// their coefficients as 16-byte vectors where their points coincide.
 template <int D, bool PAIR>
-__global__ void __launch_bounds__(kThreadsNd) eval3d_kernel(const __grid_constant__ EvalNdArgs a, int ppb, int H, int hs)
+__global__ void __launch_bounds__(kItemThreads) eval3d_kernel(const __grid_constant__ EvalNdArgs a, int ppb, int H, int hs)
 {
-    for_items(a.m, ppb, H, hs, [&](int64_t p, int h) {
-        int64_t const at = p * a.B + (PAIR ? 2 * h : h);
-        const double* const C = a.coefs + (PAIR ? 2 * h : h);
-        const double* const x = a.coords + at * 3;
-        double const x0 = __ldcs(x), x1 = __ldcs(x + 1), x2 = __ldcs(x + 2);
-        if constexpr (PAIR) {
-            double const u0 = __ldcs(x + 3), u1 = __ldcs(x + 4), u2 = __ldcs(x + 5);
-            double2 y;
-            if (x0 == u0 && x1 == u1 && x2 == u2) {
-                y = eval3d_point<D, double2>(a, x0, x1, x2, C);
-            } else {
-                y.x = eval3d_point<D, double>(a, x0, x1, x2, C);
-                y.y = eval3d_point<D, double>(a, u0, u1, u2, C + 1);
-            }
-            __stcs(reinterpret_cast<double2*>(a.out + at), y);
-        } else {
-            __stcs(a.out + at, eval3d_point<D, double>(a, x0, x1, x2, C));
-        }
-    });
+    if constexpr (PAIR) {
+        for_items<true>(a.m, ppb, H, hs, [&](bool live, int64_t p, int h) {
+            int64_t const at = p * a.B + 2 * h;
+            const double* const v = a.coords + at * 3;
+            double const x0 = __ldcs(v), x1 = __ldcs(v + 1), x2 = __ldcs(v + 2);
+            pair_items(
+                live, at, h, x0 == __ldcs(v + 3) && x1 == __ldcs(v + 4) && x2 == __ldcs(v + 5),
+                [&](int64_t to, int c) {
+                    __stcs(reinterpret_cast<double2*>(a.out + to), eval3d_point<D, double2>(a, x0, x1, x2, a.coefs + 2 * c));
+                },
+                [&](int64_t to, int field) {
+                    const double* const u = a.coords + to * 3;
+                    __stcs(a.out + to, eval3d_point<D, double>(a, __ldcs(u), __ldcs(u + 1), __ldcs(u + 2), a.coefs + field));
+                });
+        });
+    } else {
+        for_items<false>(a.m, ppb, H, hs, [&](int64_t p, int h) {
+            int64_t const at = p * a.B + h;
+            const double* const v = a.coords + at * 3;
+            __stcs(a.out + at, eval3d_point<D, double>(a, __ldcs(v), __ldcs(v + 1), __ldcs(v + 2), a.coefs + h));
+        });
+    }
 }
 
 template <int D>
 void launch_eval3d(EvalNdArgs const& a, cudaStream_t s)
 {
     bool const pair = a.B % 2 == 0 && reinterpret_cast<uintptr_t>(a.coefs) % 16 == 0 && reinterpret_cast<uintptr_t>(a.out) % 16 == 0;
-    int const H = int(pair ? a.B / 2 : a.B), hs = std::min(H, 32), ppb = kItemsNd / hs;
-    dim3 const grid((unsigned)((a.m + ppb - 1) / ppb), (unsigned)((H + hs - 1) / hs));
-    if (pair) eval3d_kernel<D, true><<<grid, kThreadsNd, 0, s>>>(a, ppb, H, hs);
-    else eval3d_kernel<D, false><<<grid, kThreadsNd, 0, s>>>(a, ppb, H, hs);
+    ItemGrid const g = item_grid(a.m, a.B, pair);
+    if (pair) eval3d_kernel<D, true><<<g.grid, kItemThreads, 0, s>>>(a, g.ppb, g.H, g.hs);
+    else eval3d_kernel<D, false><<<g.grid, kItemThreads, 0, s>>>(a, g.ppb, g.H, g.hs);
 }
 
 struct IntegrateNdArgs
@@ -448,9 +426,8 @@ void launch_evalnd(Evaluator const* const* e, int ndims, int const* orders, doub
         default: launch_eval3d<5>(a, s); break;
         }
     } else {
-        int const hs = int(std::min<int64_t>(B, 32)), ppb = kItemsNd / hs;
-        dim3 const grid((unsigned)((m + ppb - 1) / ppb), (unsigned)((B + hs - 1) / hs));
-        evalnd_kernel<<<grid, kThreadsNd, 0, s>>>(a, ppb, int(B), hs);
+        ItemGrid const g = item_grid(m, B, false);
+        evalnd_kernel<<<g.grid, kItemThreads, 0, s>>>(a, g.ppb, g.H, g.hs);
     }
     DDCB_CUDA_CHECK(cudaGetLastError());
 }
