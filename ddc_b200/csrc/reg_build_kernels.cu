@@ -80,9 +80,12 @@ bool launch_reg(BuildArgs const& args, cudaStream_t s)
     // loads and stores beside the other's sweeps (513 rows x 32768 lines: 63 us against 78 in one
     // block of 32 lines); else one block of up to 512 threads with the widest tile (1027 rows x
     // 65536 lines: 241 us with 16 lines against 320 in two blocks of 8).
-    // Unit-stride lines read the same segments with any width: two blocks of eight lines.
+    // Unit-stride lines read the same segments with any width: two blocks of eight lines; of sixteen
+    // where eight would leave most of a warp without a chunk, or with a border to wait for (Greville
+    // cubics x 65536 lines, 32 cells in 2 chunks: 37 us against 41; x 16384 lines, 100 cells in 6 chunks
+    // and 4 border rows: 21 against 27; but without a border, 64 cells in 4 chunks: 33 against 27).
     bool const staged = io.stage_out || (args.lv.stride == 1 && args.lv.inner == 1 && args.lv.outer > 1);
-    io.lp = staged ? 2 : 5;
+    io.lp = !staged ? 5 : (t.nchunk <= 2 || (t.nchunk <= 6 && t.k >= 4) ? 3 : 2);
     while (io.lp > 3 && !fits(256, 2)) --io.lp;
     if (!fits(256, 2)) {
         io.lp = 5;

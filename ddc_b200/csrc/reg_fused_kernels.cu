@@ -107,8 +107,12 @@ bool launch_reg_fused_kd(BuildArgs const& args, FusedEval const& fe, cudaStream_
     auto tiles = [&] { return (args.nlines + (int64_t(2) << io.lp) - 1) >> (io.lp + 1); };
     // Two blocks of 256 threads per SM, one's copies beside the other's evaluation, with tiles of
     // eight lines or more; else one block of 512. A batch that leaves SMs without a tile takes
-    // narrower tiles down to eight lines, and 512 threads to evaluate each.
-    io.lp = 4;
+    // narrower tiles down to eight lines, and 512 threads to evaluate each. Unit-stride points want eight
+    // lines too, so that a warp's segments of a line are whole sectors (512 cells x 16384 lines: 117 us
+    // against 163 with 16 lines), unless the lines have so few chunks that the solve would keep but a warp
+    // of the block (100 cells: 61 against 40).
+    bool const unit = fe.lo.stride == 1 && fe.lo.inner == 1 && fe.lo.outer > 1;
+    io.lp = unit && t.nchunk >= 16 ? 2 : 4;
     while (io.lp > 2 && (!fits(256, 2) || tiles() < int64_t(sms))) --io.lp;
     int threads = 256;
     if (!fits(256, 2) || tiles() <= int64_t(sms)) threads = 512;
