@@ -12,6 +12,7 @@ struct AdjointArgs
     RhsMap r;
     int64_t nlines;
     int nct;
+    int tile_req;           // Builder::tile_req
     const double* gc;       // cotangents of the coefficients (size rows)
     Lines lgc;
     double* gv;             // cotangents of the samples (npoints rows)

@@ -426,6 +426,7 @@ AdjointArgs make_adjoint_args(Builder const& b, const double* gc, Lines const& l
     AdjointArgs a {};
     a.t = b.tables_t;
     a.r = b.rhs;
+    a.tile_req = b.tile_req;
     a.nlines = lgv.nlines();
     a.gc = gc;
     a.lgc = lgc;

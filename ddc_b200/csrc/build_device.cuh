@@ -44,7 +44,16 @@ struct BuildArgs
     int pair16;         // vals: adjacent line pairs are 16-byte aligned and contiguous
     int pair16_out;     // out: the same for the coefficient output
     int64_t line_base;  // first line of the block's tile; < 0: blockIdx.x * TL
+    int tile_req;       // Builder::tile_req
 };
+
+// log2 of the line pairs a block of the register solve may take: as requested, at most 2^5.
+inline int most_pairs(int tile_req)
+{
+    int lp = 5;
+    while (tile_req > 0 && lp > 0 && (2 << lp) > tile_req) --lp;
+    return lp;
+}
 
 // First line of the block's tile.
 template <int TL>

@@ -121,6 +121,7 @@ BuildArgs make_build_args(Builder const& b, double* coefs, Lines const& lc, doub
     args.out = coefs;
     args.lo = lc;
     args.nct = pick_nct(b.tables, b.tile_lines);
+    args.tile_req = b.tile_req;
     args.pair16 = line_pairs_aligned(vals, lv);
     args.pair16_out = line_pairs_aligned(coefs, lc);
     return args;
@@ -213,6 +214,7 @@ void launch_build(Builder const& b, double* coefs, Lines const& lc, double const
     args.out = coefs;
     args.lo = lc;
     args.nct = pick_nct(b.tables, b.tile_lines);
+    args.tile_req = b.tile_req;
     args.pair16 = line_pairs_aligned(vals, lv);
     args.pair16_out = line_pairs_aligned(coefs, lc);
     if (args.nlines == 0) return;
@@ -249,6 +251,7 @@ void launch_solve_multirhs(Builder const& b, double* rhs, long ld, long nrhs, bo
     args.out = rhs;
     args.lo = L;
     args.nct = pick_nct(args.t, b.tile_lines);
+    args.tile_req = b.tile_req;
     args.pair16 = args.pair16_out = line_pairs_aligned(rhs, L);
     if (nrhs == 0) return;
     if (launch_reg_build(args, s)) return;

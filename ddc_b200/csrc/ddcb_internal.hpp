@@ -240,6 +240,7 @@ struct Builder
     double refine_tolerance = 1e-12; // bound on ||A^-1|| |b - A x| / |x| after the last round
     int device = -1;
     int tile_lines = 8;     // lines per CTA
+    int tile_req = 0;       // requested lines per CTA (0: the register solve picks its own by the batch)
     int nchunk_req = 0;     // requested chunks per line (0: chosen by the plan, HostSolve::make_tables)
     // host copies of the solve tables (for quadrature / transposed host solves)
     int k = 0, m = 0, kl = 0, ku = 0, pivot = 0;

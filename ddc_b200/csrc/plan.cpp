@@ -1182,7 +1182,7 @@ Builder* create_builder_host(Basis const& basis, double const* pts, long npts, i
             if (opts->refine_rounds > 0) b->refine_rounds = opts->refine_rounds;
             if (!(opts->refine_tolerance >= 0.0)) throw Error(DDCB_ERR_INVALID_ARGUMENT, "refine_tolerance must be >= 0");
             if (opts->refine_tolerance > 0.0) b->refine_tolerance = opts->refine_tolerance;
-            if (opts->tile_lines > 0) b->tile_lines = opts->tile_lines;
+            if (opts->tile_lines > 0) b->tile_req = b->tile_lines = opts->tile_lines;
             if (opts->chunks > 0) b->nchunk_req = opts->chunks;
         }
         if (b->tile_lines != 2 && b->tile_lines != 4 && b->tile_lines != 8 && b->tile_lines != 16)

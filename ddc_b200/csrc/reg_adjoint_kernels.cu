@@ -231,7 +231,7 @@ bool launch_kd(AdjointArgs const& a, EvalAdjointArgs const& ea, cudaStream_t s)
     int const v0 = a.r.periodic ? 0 : a.r.nbe_lo, v1 = a.r.periodic ? t.n : a.r.nbe_lo + a.r.npoints;
     if (a.r.lrot < v0 || a.r.lrot + t.m > v1 || ea.lx.n > (int64_t(1) << 30)) return false;
     int const optin = device_limits().optin, sms = device_limits().sms;
-    int lp = 3;
+    int lp = std::min(most_pairs(a.tile_req), 3);
     auto bytes = [&] { return sizeof(double) * (reg_smem_doubles<K>(t, 1 << lp) + size_t(t.n + ea.size) * size_t(2 << lp)); };
     auto fits = [&](int threads, int blocks) { return (t.nchunk << lp) <= threads && bytes() + 1024 <= (size_t(optin) + 1024) / blocks; };
     auto tiles = [&] { return (a.nlines + (int64_t(2) << lp) - 1) >> (lp + 1); };

@@ -85,10 +85,11 @@ bool launch_reg(BuildArgs const& args, cudaStream_t s)
     // cubics x 65536 lines, 32 cells in 2 chunks: 37 us against 41; x 16384 lines, 100 cells in 6 chunks
     // and 4 border rows: 21 against 27; but without a border, 64 cells in 4 chunks: 33 against 27).
     bool const staged = io.stage_out || (args.lv.stride == 1 && args.lv.inner == 1 && args.lv.outer > 1);
-    io.lp = !staged ? 5 : (t.nchunk <= 2 || (t.nchunk <= 6 && t.k >= 4) ? 3 : 2);
+    int const most = most_pairs(args.tile_req);
+    io.lp = std::min(most, !staged ? 5 : (t.nchunk <= 2 || (t.nchunk <= 6 && t.k >= 4) ? 3 : 2));
     while (io.lp > 3 && !fits(256, 2)) --io.lp;
     if (!fits(256, 2)) {
-        io.lp = 5;
+        io.lp = most;
         while (io.lp > 0 && !fits(512, 1)) --io.lp;
     }
     while (io.lp > 1 && tiles() < int64_t(sms)) --io.lp; // at least a block for every SM

@@ -112,7 +112,7 @@ bool launch_reg_fused_kd(BuildArgs const& args, FusedEval const& fe, cudaStream_
     // against 163 with 16 lines), unless the lines have so few chunks that the solve would keep but a warp
     // of the block (100 cells: 61 against 40).
     bool const unit = fe.lo.stride == 1 && fe.lo.inner == 1 && fe.lo.outer > 1;
-    io.lp = unit && t.nchunk >= 16 ? 2 : 4;
+    io.lp = std::min(most_pairs(args.tile_req), unit && t.nchunk >= 16 ? 2 : 4);
     while (io.lp > 2 && (!fits(256, 2) || tiles() < int64_t(sms))) --io.lp;
     int threads = 256;
     if (!fits(256, 2) || tiles() <= int64_t(sms)) threads = 512;
