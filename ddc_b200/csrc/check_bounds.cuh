@@ -8,7 +8,9 @@
 // unit (the first event per query wins: the site's file and line, the index and the bound) and the
 // kernel goes on with the index clamped into range: no trap, no device assert, no access outside
 // the array. ddcb_last_device_error reads and clears the words of every translation unit. In the
-// default build DDCB_INDEX is the index itself.
+// default build DDCB_INDEX is the index itself. Loops that walk a pointer from row to row name the row
+// it stands at: DDCB_ROW(p, base, i, n, stride) is the pointer p there, and base + (checked i) * stride
+// in the checked build.
 #pragma once
 
 #include <cstdint>
@@ -85,9 +87,11 @@ BoundsRegistration const g_bounds_registration;
     static_cast<decltype(i)>(::ddcb::bounds_checked(static_cast<long long>(i), static_cast<long long>(n),       \
                                                     (static_cast<unsigned long long>(::ddcb::bounds_file_tag(__FILE__)) << 16) | \
                                                         static_cast<unsigned long long>(__LINE__)))
+#define DDCB_ROW(p, base, i, n, stride) ((base) + static_cast<long long>(DDCB_INDEX(i, n)) * (stride))
 
 #else
 
 #define DDCB_INDEX(i, n) (i)
+#define DDCB_ROW(p, base, i, n, stride) (p)
 
 #endif

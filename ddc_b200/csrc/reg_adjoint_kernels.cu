@@ -87,10 +87,11 @@ __device__ __forceinline__ void reg_store_samples(AdjointArgs const& a, int64_t 
     if (line >= a.nlines) return;
     int64_t const st = a.lgv.stride;
     double* g = a.gv + first * st + line_offset(a.lgv, line);
+    [[maybe_unused]] double* const base = a.gv + line_offset(a.lgv, line);
     if (a.pair_out) {
 #pragma unroll
         for (int s = 0; s < kRegRows; ++s) {
-            if (s < len) __stcs(reinterpret_cast<double2*>(g), x[s]);
+            if (s < len) __stcs(reinterpret_cast<double2*>(DDCB_ROW(g, base, first + s, a.r.npoints, st)), x[s]);
             g += st;
         }
         return;
@@ -100,8 +101,9 @@ __device__ __forceinline__ void reg_store_samples(AdjointArgs const& a, int64_t 
 #pragma unroll
     for (int s = 0; s < kRegRows; ++s) {
         if (s < len) {
-            __stcs(g, x[s].x);
-            if (two) __stcs(g + next, x[s].y);
+            double* const to = DDCB_ROW(g, base, first + s, a.r.npoints, st);
+            __stcs(to, x[s].x);
+            if (two) __stcs(to + next, x[s].y);
         }
         g += st;
     }

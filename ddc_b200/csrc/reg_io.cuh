@@ -41,7 +41,7 @@ __device__ __forceinline__ const double* border_source(BuildArgs const& args, in
     int const v0 = all ? 0 : R.nbe_lo, v1 = all ? n : R.nbe_lo + R.npoints;
     int sr = args.t.m + r + R.lrot;
     sr -= (sr >= n) ? n : 0;
-    if (sr >= v0 && sr < v1) return args.vals + (int64_t)(sr - v0) * args.lv.stride + line_offset(args.lv, line);
+    if (sr >= v0 && sr < v1) return args.vals + (int64_t)DDCB_INDEX(sr - v0, v1 - v0) * args.lv.stride + line_offset(args.lv, line);
     if (sr < R.nbe_lo) return sr < R.nbv_lo ? args.dlo + sr * args.llo.stride + line_offset(args.llo, line) : nullptr;
     int const i = sr - (n - R.nbe_hi);
     return i < R.nbv_hi ? args.dhi + i * args.lhi.stride + line_offset(args.lhi, line) : nullptr;
@@ -66,7 +66,9 @@ __device__ __forceinline__ void reg_fill(BuildArgs const& args, RegIo const& io,
     int const TL = 2 << io.lp;
     int const m = args.t.m;
     int64_t const st = args.lv.stride;
-    const double* const vals = args.vals + (int64_t)(args.r.lrot - io.v0) * st;
+    int const first = args.r.lrot - io.v0; // the sample of row 0
+    const double* const vals = args.vals + (int64_t)first * st;
+    [[maybe_unused]] int const samples = args.raw ? args.t.n : args.r.npoints;
     if (args.pair16) {
         int const P = 1 << io.lp;
         int const p = threadIdx.x & (P - 1);
@@ -77,7 +79,7 @@ __device__ __forceinline__ void reg_fill(BuildArgs const& args, RegIo const& io,
         int64_t const gs = step * st;
         double* s = tile + r0 * TL + 2 * p;
         for (int r = r0; r < m; r += step) {
-            cp_async16(s, g);
+            cp_async16(s, DDCB_ROW(g, args.vals + line_offset(args.lv, line), first + r, samples, st));
             g += gs;
             s += step * TL;
         }
@@ -91,7 +93,7 @@ __device__ __forceinline__ void reg_fill(BuildArgs const& args, RegIo const& io,
         int64_t const gs = step * st;
         double* s = tile + r0 * TL + l;
         for (int r = r0; r < m; r += step) {
-            cp_async8(s, g);
+            cp_async8(s, DDCB_ROW(g, args.vals + line_offset(args.lv, line), first + r, samples, st));
             g += gs;
             s += step * TL;
         }
@@ -154,7 +156,7 @@ __device__ __forceinline__ void reg_store_tile(BuildArgs const& args, RegIo cons
 #pragma unroll
     for (int s = 0; s < kRegRows; ++s)
         if (s < len) {
-            int const q = o + s - (o + s >= n ? n : 0);
+            int const q = DDCB_INDEX(o + s - (o + s >= n ? n : 0), n);
             *reinterpret_cast<double2*>(t0 + q * TL) = x[s];
             if (q < dup) *reinterpret_cast<double2*>(t0 + (q + n) * TL) = x[s];
         }
@@ -179,15 +181,16 @@ __device__ __forceinline__ void reg_store(BuildArgs const& args, int64_t line, i
         if (args.pair16_out) {
 #pragma unroll
             for (int s = 0; s < R; ++s) {
-                if (s < len) __stcs(reinterpret_cast<double2*>(g), x[s]);
+                if (s < len) __stcs(reinterpret_cast<double2*>(DDCB_ROW(g, base, o + s, n, st)), x[s]);
                 g += st;
             }
         } else {
 #pragma unroll
             for (int s = 0; s < R; ++s) {
                 if (s < len) {
-                    __stcs(g, x[s].x);
-                    if (two) __stcs(g + next, x[s].y);
+                    double* const to = DDCB_ROW(g, base, o + s, n, st);
+                    __stcs(to, x[s].x);
+                    if (two) __stcs(to + next, x[s].y);
                 }
                 g += st;
             }
@@ -197,7 +200,7 @@ __device__ __forceinline__ void reg_store(BuildArgs const& args, int64_t line, i
 #pragma unroll
     for (int s = 0; s < R; ++s)
         if (s < len) {
-            int const q = o + s - (o + s >= n ? n : 0);
+            int const q = DDCB_INDEX(o + s - (o + s >= n ? n : 0), n);
             double* const g = base + (int64_t)q * st;
             double* const g2 = q < dup ? g + n * st : g;
             if (args.pair16_out) {

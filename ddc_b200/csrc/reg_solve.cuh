@@ -210,13 +210,13 @@ __device__ __forceinline__ void reg_border(SolveTables const& t, RegSmem const& 
 #pragma unroll
         for (int s = 0; s < kRegRows; ++s) {
             if (a + s >= lo || s >= len) break;
-            E[(a + s) * P] = x[s];
+            E[DDCB_INDEX(a + s, lo + t.lam_hi) * P] = x[s];
         }
 #pragma unroll
         for (int s = kRegRows - 1; s >= 0; --s) {
             if (s >= len) continue;
             if (a + s < hi0) break;
-            if (a + s >= lo) E[(lo + a + s - hi0) * P] = x[s];
+            if (a + s >= lo) E[DDCB_INDEX(lo + a + s - hi0, lo + t.lam_hi) * P] = x[s];
         }
     }
     __syncthreads();
@@ -232,7 +232,7 @@ __device__ __forceinline__ void reg_border(SolveTables const& t, RegSmem const& 
             double2 s = b2[r * P];
             int const j1 = lam_row[r + 1];
 #pragma unroll 4
-            for (int j = lam_row[r]; j < j1; ++j) s = fma2(-lam[j], sm.ends[lam_end[j] * P + q], s);
+            for (int j = lam_row[r]; j < j1; ++j) s = fma2(-lam[j], sm.ends[DDCB_INDEX(lam_end[j], t.lam_lo + t.lam_hi) * P + q], s);
             b2[r * P] = s;
         }
         __syncwarp(lanes);
@@ -246,7 +246,7 @@ __device__ __forceinline__ void reg_border(SolveTables const& t, RegSmem const& 
     __syncthreads();
     int const e = c < t.cor_lo ? c : c - (t.nchunk - nc);
     if (c < t.nchunk && (c < t.cor_lo || c >= t.nchunk - t.cor_hi)) {
-        const double* g = sm.bord + e * k * W;
+        const double* g = sm.bord + DDCB_INDEX(e, nc) * k * W;
 #pragma unroll 1
         for (int r = 0; r < k; ++r, g += W) {
             double2 const v = sm.x2[r * P + p];
