@@ -1066,7 +1066,15 @@ ddcb_status ddcb_build2d(ddcb_builder h1, ddcb_builder h2, double* coefs, const 
         bool owned = false;
         int64_t group = 0; // as many fields at once as the build likes
         if (ws == nullptr) {
-            DDCB_CUDA_CHECK(cudaMallocAsync(&ws, need, s));
+            // where there is no room for the widest groups, those that a caller's smallest workspace holds
+            cudaError_t got = cudaMallocAsync(&ws, need, s);
+            if (got == cudaErrorMemoryAllocation) {
+                cudaGetLastError();
+                size_t const least = ddcb::build2d_least_workspace_bytes(b1, b2, nbatch);
+                got = cudaMallocAsync(&ws, least, s);
+                group = ddcb::build2d_group_for(b1, b2, nbatch, least);
+            }
+            DDCB_CUDA_CHECK(got);
             owned = true;
         } else if (workspace_bytes < need) { // smaller groups of fields in a smaller workspace
             group = ddcb::build2d_group_for(b1, b2, nbatch, workspace_bytes);

@@ -391,6 +391,7 @@ struct SideStream
 };
 SideStream& side_stream_for_current_device();
 size_t build2d_workspace_bytes(Builder const& b1, Builder const& b2, int64_t nbatch);
+size_t build2d_least_workspace_bytes(Builder const& b1, Builder const& b2, int64_t nbatch);
 int64_t build2d_group_for(Builder const& b1, Builder const& b2, int64_t nbatch, size_t bytes);
 void launch_build2d(Builder const& b1, Builder const& b2, double* coefs, double const* vals, double const* dmin1,
                     double const* dmax1, double const* dmin2, double const* dmax2, double const* m11, double const* m21,

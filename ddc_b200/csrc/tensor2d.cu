@@ -71,8 +71,13 @@ size_t build2d_workspace_bytes(Builder const& b1, Builder const& b2, int64_t nba
     return workspace_for_group(b1, b2, nbatch, group_fields(b1, b2, nbatch));
 }
 
-// The widest group whose workspace fits in `bytes`; 0 below the workspace of the L2-sized group, which
-// is the least a caller has to bring.
+// The least a caller has to bring: the workspace of the L2-sized group.
+size_t build2d_least_workspace_bytes(Builder const& b1, Builder const& b2, int64_t nbatch)
+{
+    return workspace_for_group(b1, b2, nbatch, std::min(group_fields(b1, b2, nbatch), l2_fields(b1, b2)));
+}
+
+// The widest group whose workspace fits in `bytes`; 0 below that.
 int64_t build2d_group_for(Builder const& b1, Builder const& b2, int64_t nbatch, size_t bytes)
 {
     int64_t G = group_fields(b1, b2, nbatch);
