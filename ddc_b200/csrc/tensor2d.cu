@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(kItemThreads) eval2d_kernel(const __grid_const
         for_items<true>(a.m, ppb, H, hs, [&](bool live, int64_t p, int h) {
             int64_t const at = p * a.B + 2 * h;
             double2 const u = __ldcs(xy + at), w = __ldcs(xy + at + 1);
-            pair_items(
+            pair_items<U1 && U2 ? 2 : 1>(
                 live, at, h, u.x == w.x && u.y == w.y,
                 [&](int64_t to, int c) {
                     __stcs(reinterpret_cast<double2*>(a.out + to),

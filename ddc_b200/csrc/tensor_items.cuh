@@ -20,7 +20,7 @@ struct ItemGrid
     dim3 grid;
 };
 
-// 32 fields a block at most, so that the blocks in flight gather from as many: all 64 quintic fields of
+// Some 32 fields a block, so that the blocks in flight gather from as many: all 64 quintic fields of
 // 512^2 do not fit the L2 (30000 points, each field its own: 343 us with 16 columns, 520 with 32). A
 // thread takes one item until every SM has eight blocks, then two. In blocks of 2048 items, whatever
 // the batch, one cubic field of 48^3 at 7000 points took 49 us (13 now) and 64 fields of 512^2 at
@@ -29,7 +29,9 @@ inline ItemGrid item_grid(int64_t m, int64_t B, bool pair)
 {
     ItemGrid g;
     g.H = int(pair ? B / 2 : B);
-    g.hs = std::min(g.H, pair && g.H <= 16 * 65535 ? 16 : 32); // (the grid's second dimension ends there)
+    int const most = pair && g.H <= 16 * 65535 ? 16 : 32; // (the grid's second dimension ends there)
+    int const groups = std::max(1, (g.H + most / 2 - 1) / most); // equal ones: 33 columns are one group, not 32 and 1
+    g.hs = (g.H + groups - 1) / groups;
     int64_t const each = (m * g.H + 8 * device_limits().sms - 1) / (8 * device_limits().sms);
     int64_t const items = std::min<int64_t>(kMostItems, std::max<int64_t>(1, (each + kItemThreads - 1) / kItemThreads) * kItemThreads);
     g.ppb = int(items) / g.hs;
@@ -65,8 +67,11 @@ __device__ __forceinline__ void for_items(int64_t m, int ppb, int H, int hs, F f
 // The items of a warp over pairs of fields. Where all pairs share their point, a lane takes a pair: one
 // basis, 16-byte loads. Where not, neighbouring lanes take the two fields of a pair, half of the warp's
 // pairs after the other, so that a request still reads neighbouring fields. `at`: where the pair's first
-// value goes; `shared`: whether its points coincide; one(to, field), both(at, column).
-template <class Both, class One>
+// value goes; `shared`: whether its points coincide; one(to, field), both(at, column). UNROLL: the two
+// halves' code side by side, 2 where its registers allow (uniform cubics: 64 fields on a displaced mesh
+// of their own 207 us against 215, on a shared one 147 against 155; but irregular cubics, 64 fields at
+// 30000 shared points, 55 against 45).
+template <int UNROLL, class Both, class One>
 __device__ __forceinline__ void pair_items(bool live, int64_t at, int h, bool shared, Both both, One one)
 {
     constexpr unsigned kAll = 0xffffffffu;
@@ -76,7 +81,7 @@ __device__ __forceinline__ void pair_items(bool live, int64_t at, int h, bool sh
     }
     int const lane = threadIdx.x & 31;
     at = live ? at : -1;
-#pragma unroll 1
+#pragma unroll UNROLL
     for (int half = 0; half < 32; half += 16) {
         int64_t const to = __shfl_sync(kAll, at, half + lane / 2);
         int const c = __shfl_sync(kAll, h, half + lane / 2);

@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(kItemThreads) eval3d_kernel(const __grid_const
             int64_t const at = p * a.B + 2 * h;
             const double* const v = a.coords + at * 3;
             double const x0 = __ldcs(v), x1 = __ldcs(v + 1), x2 = __ldcs(v + 2);
-            pair_items(
+            pair_items<D <= 3 ? 2 : 1>(
                 live, at, h, x0 == __ldcs(v + 3) && x1 == __ldcs(v + 4) && x2 == __ldcs(v + 5),
                 [&](int64_t to, int c) {
                     __stcs(reinterpret_cast<double2*>(a.out + to), eval3d_point<D, double2>(a, x0, x1, x2, a.coefs + 2 * c));
