@@ -1229,10 +1229,12 @@ Builder* create_builder_host(Basis const& basis, double const* pts, long npts, i
             rows.swap(rot);
         }
         priv->fwd.analyse(rows, D.periodic != 0, top + bottom);
-        // the refined solve works in the shared-memory tile, whose threads the chunks are; the long
-        // chunks of the register solve would leave it a fraction of them (256 cells x 1000 lines,
-        // quintic: 86 us against 33 with 64 chunks)
-        priv->fwd.make_tables(b->nchunk_req == 0 && b->precision == DDCB_FP32_REFINE ? kTileChunks : b->nchunk_req);
+        // the refined solve works in the shared-memory tile, whose threads the chunks are: on lines that
+        // the register solve cuts into fewer than 64, its long chunks would leave a fraction of them
+        // (256 cells x 1000 lines, quintic: 86 us against 35 with 64 chunks; but 2000 cells x 4096
+        // lines, cubic, 117 chunks: 300 against 446)
+        bool const tile = b->precision == DDCB_FP32_REFINE && priv->fwd.m <= kTileChunks * kRegRows;
+        priv->fwd.make_tables(b->nchunk_req == 0 && tile ? kTileChunks : b->nchunk_req);
         priv->adj.analyse(transpose_rows(rows), D.periodic != 0, top + bottom);
         priv->adj.make_tables(b->nchunk_req);
         b->k = int(priv->fwd.k);
