@@ -83,8 +83,10 @@ typedef struct ddcb_bsplines_info {
 typedef struct ddcb_builder_options {
     int32_t precision;       /* ddcb_precision */
     int32_t refine_rounds;   /* FP32_REFINE: refinement rounds (1..3; 0 = 2) */
-    int32_t tile_lines;      /* 0 = automatic: lines per thread block */
-    int32_t chunks;          /* 0 = automatic: chunk threads per line */
+    int32_t tile_lines;      /* 2, 4, 8 or 16: the most lines per thread block; 0 = automatic (by the batch,
+                                or 8 where lines are solved in a shared-memory tile) */
+    int32_t chunks;          /* chunk threads per line; 0 = automatic (as few as a thread's registers hold,
+                                64 for longer lines and for FP32_REFINE up to 1088 rows) */
     double refine_tolerance; /* FP32_REFINE: bound on the estimated relative error of a refined line,
                                 ||A^-1||_inf max|b - A x| / max|x| after the last round, checked on
                                 the device (0 = 1e-12); see ddcb_builder_device_status */
@@ -95,7 +97,7 @@ typedef struct ddcb_builder_info {
     int32_t nbe_lo, nbe_hi, nbv_lo, nbv_hi; /* s_nbe_xmin/xmax, s_nbv_xmin/xmax (spline_builder.hpp:166-191) */
     int32_t offset;                         /* m_offset (spline_builder.hpp:201, 619-658) */
     double dx;                              /* m_dx (spline_builder.hpp:233-234) */
-    int32_t border, kl, ku, pivoting, chunks, tile_lines; /* structure of the device solve */
+    int32_t border, kl, ku, pivoting, chunks, tile_lines; /* structure of the device solve (tile_lines 8 where it was left automatic) */
 } ddcb_builder_info;
 
 /* ---- status ---------------------------------------------------------------------------- */
