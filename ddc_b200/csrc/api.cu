@@ -4,8 +4,10 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <map>
 #include <mutex>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include <nvtx3/nvToolsExt.h>
@@ -34,6 +36,21 @@ DeviceLimits const& device_limits()
         limits[dev] = l;
     });
     return limits[dev];
+}
+
+// The most any launch of this process has asked for, which every launch sets again. (With all that the
+// device has as every kernel's limit, calls of a few lines took 11.1 us instead of 10.7.)
+void allow_shared(const void* kern, size_t bytes)
+{
+    static std::mutex mutex;
+    static auto* const most = new std::map<std::pair<int, const void*>, size_t>; // (outlives late callers)
+    int dev = 0;
+    DDCB_CUDA_CHECK(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lock(mutex); // until the limit is set: a lower one must not come after it
+    size_t& m = (*most)[{dev, kern}];
+    size_t const limit = std::max(m, bytes);
+    DDCB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(limit)));
+    m = limit;
 }
 
 } // namespace ddcb

@@ -36,16 +36,15 @@ struct DeviceLimits
 };
 DeviceLimits const& device_limits();
 
+// Lets `kern` take `bytes` of dynamic shared memory on the current device (api.cu). The limit belongs to
+// the kernel on the device, not to the launch that sets it, so it is only ever raised: a small launch
+// of another host thread, between this call and the launch it is for, must not lower it.
+void allow_shared(const void* kern, size_t bytes);
 #if defined(__CUDACC__)
-// Lets `kern` take `bytes` of dynamic shared memory. The limit belongs to the kernel on the device,
-// not to the launch that sets it: every launch that needs one sets the same, the most the kernel can
-// have beside its `fixed` static bytes, so that a small launch of another host thread, between this
-// call and the launch it is for, cannot lower it.
 template <class Kern>
-void allow_shared(Kern kern, size_t bytes, size_t fixed = 0)
+void allow_shared(Kern kern, size_t bytes)
 {
-    if (bytes > 48 * 1024)
-        DDCB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(size_t(device_limits().optin) - fixed)));
+    if (bytes > 48 * 1024) allow_shared(reinterpret_cast<const void*>(kern), bytes);
 }
 #endif
 

@@ -290,9 +290,7 @@ int group_blocks(UnevenBatch const& b, int g, int threads, int per_sm)
 {
     UnevenKernel k = kernel_of(b.gshape[size_t(g)], b.grefine[size_t(g)] != 0);
     size_t const sm = b.gsmem[size_t(g)];
-    cudaFuncAttributes fa {};
-    DDCB_CUDA_CHECK(cudaFuncGetAttributes(&fa, k));
-    allow_shared(k, sm, fa.sharedSizeBytes);
+    allow_shared(k, sm);
     int fit = 0;
     DDCB_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, k, threads, sm));
     if (fit < 1) throw Error(DDCB_ERR_UNSUPPORTED, "the largest problem's tile does not fit in shared memory");
