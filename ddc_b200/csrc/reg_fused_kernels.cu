@@ -110,8 +110,9 @@ bool launch_reg_fused_kd(BuildArgs const& args, FusedEval const& fe, cudaStream_
     // narrower tiles down to eight lines, and 512 threads to evaluate each. Unit-stride points want eight
     // lines too, so that a warp's segments of a line are whole sectors (512 cells x 16384 lines: 117 us
     // against 163 with 16 lines), unless the lines have so few chunks that the solve would keep but a warp
-    // of the block (100 cells: 61 against 40).
-    bool const unit = fe.lo.stride == 1 && fe.lo.inner == 1 && fe.lo.outer > 1;
+    // of the block (100 cells: 61 against 40). Feet are not read: sixteen lines (Greville cubics: 95
+    // against 99).
+    bool const unit = !FEET && fe.lo.stride == 1 && fe.lo.inner == 1 && fe.lo.outer > 1;
     io.lp = std::min(most_pairs(args.tile_req), unit && t.nchunk >= 16 ? 2 : 4);
     while (io.lp > 2 && (!fits(256, 2) || tiles() < int64_t(sms))) --io.lp;
     int threads = 256;
